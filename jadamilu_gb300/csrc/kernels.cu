@@ -213,12 +213,12 @@ template <class T> void fill(long n, T v, T* x, cudaStream_t s) {
 }
 
 // ---------------------------------------------------- reductions (V^H w) ----
-__device__ __forceinline__ double shfl_down(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ zc shfl_down(zc v, int o) { return zc(shfl_down(v.x, o), shfl_down(v.y, o)); }
 __device__ __forceinline__ float shfl_xor_any(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ double shfl_xor_any(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ cc shfl_xor_any(cc v, int o) { return cc(shfl_xor_any(v.x, o), shfl_xor_any(v.y, o)); }
 __device__ __forceinline__ zc shfl_xor_any(zc v, int o) { return zc(shfl_xor_any(v.x, o), shfl_xor_any(v.y, o)); }
+__device__ __forceinline__ double shfl_idx_any(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+__device__ __forceinline__ zc shfl_idx_any(zc v, int l) { return zc(shfl_idx_any(v.x, l), shfl_idx_any(v.y, l)); }
 
 // loads that bypass L1 (data another CTA of the same launch wrote)
 __device__ __forceinline__ double ldcg_(const double* p) { return __ldcg(p); }
@@ -227,7 +227,9 @@ __device__ __forceinline__ zc ldcg_(const zc* p) {
   return zc(v.x, v.y);
 }
 
-constexpr int MD_CH = 8;  // columns per pass
+constexpr int MD_CH = 8;       // columns per group (one grid row of CTAs)
+constexpr int MD_GROUPS = 16;  // column groups of one call: k <= 128
+constexpr int MD_WARPS = TPB / 32;
 // Long vectors: up to two rows per thread, enough CTAs in flight to stream V
 // at full bandwidth.  Vectors under 4096 rows keep one CTA per 2048 rows, the
 // summation order validated on the user-guide samples (n = 1000), whose JD
@@ -237,79 +239,139 @@ static inline int md_grid(long n) {
   return (int)std::min<long>((n + 511) / 512, 152L * 8);
 }
 
-// The partials follow a 16-byte arrival counter at the start of the buffer
-// (zero when the buffer is allocated; the last CTA of each call resets it).
-constexpr int MD_HEAD = 16;
+// The partials follow one arrival counter per column group at the start of
+// the buffer (zero when the buffer is allocated; the last CTA of a group
+// resets its counter).
+constexpr int MD_HEAD = MD_GROUPS * (int)sizeof(unsigned);
 long mdot_partial_size(long n, int k) {
-  return (long)md_grid(n) * ((k + MD_CH - 1) / MD_CH) * MD_CH + 2;  // + the counter (2 doubles or 1 complex)
+  return (long)md_grid(n) * ((k + MD_CH - 1) / MD_CH) * MD_CH + MD_HEAD / (long)sizeof(double);
 }
 
-// V^H w in one launch: every CTA writes its per-column partial sums, and the
-// CTA that arrives last (a counter, no waiting) adds them per column in the
-// fixed order of a second pass (strided over TPB threads, then the warp tree),
-// so the result does not depend on which CTA is last.
-template <class T>
+// The warp tree (lane pairs 16, 8, 4, 2, 1 apart) of CH values per lane (CH a
+// power of two).  The first steps halve the columns a lane carries instead of
+// repeating the whole tree per column (CH = 8: 9 exchanges instead of 40, the
+// same pairs added).  The sum of column md_col<CH>(lane) ends in the lanes
+// whose lowest bits (lane % (32 / CH)) are zero.
+template <class T, int CH> __device__ __forceinline__ T md_tree(T (&v)[CH], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int h = CH / 2; h > 0; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < CH / 2; ++j)
+      if (j < h) {
+        const T send = up ? v[j] : v[j + h];
+        v[j] = (up ? v[j + h] : v[j]) + shfl_xor_any(send, o);
+      }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) v[0] += shfl_xor_any(v[0], o);
+  return v[0];
+}
+template <int CH> __device__ __forceinline__ int md_col(int lane) {
+  static_assert(CH == 1 || CH == 2 || CH == 8, "column groups of 1, 2 or 8");
+  return CH == 1 ? 0 : CH == 2 ? (lane >> 4) & 1 : ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+}
+
+// The end of a reduction whose threads hold CH partial sums each: a column's
+// sums go up the warp tree, then over the CTA's warps in order; the CTA of the
+// group that arrives last (a counter, no waiting) adds the CTAs' partials, one
+// warp per column.  The order is that of TPB threads striding over the g
+// partials (32 s + lane, step TPB, for s = 0 .. 7), the warp tree of each s,
+// then s in order, so the result does not depend on which CTA is last.  This
+// tail bounds the short reductions: one CTA going through the columns one by
+// one with two barriers each took 12 to 50 us a call (n = 8000: 12.1 us with
+// 25 columns at most), and the groups finish side by side.
+// Returns true in the CTA that wrote the group's results.
+template <class T, int CH>
+__device__ __forceinline__ bool md_finish(T (&acc)[CH], int nc, int c0, unsigned char* buf, T* out) {
+  __shared__ T red[MD_WARPS][CH];
+  __shared__ bool last;
+  unsigned* count = reinterpret_cast<unsigned*>(buf) + blockIdx.y;
+  T* partial = reinterpret_cast<T*>(buf + MD_HEAD);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = gridDim.x;
+  const T v = md_tree(acc, lane);
+  if (lane % (32 / CH) == 0) red[wid][md_col<CH>(lane)] = v;
+  __syncthreads();
+  if (threadIdx.x < nc) {
+    T t = T(0);
+#pragma unroll
+    for (int q = 0; q < MD_WARPS; ++q) t += red[q][threadIdx.x];
+    if (g == 1) out[c0 + threadIdx.x] = t;
+    else partial[(long)(c0 + threadIdx.x) * g + blockIdx.x] = t;
+  }
+  if (g == 1) return true;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(count, 1u) == (unsigned)g - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return false;
+  if (wid < nc) {
+    const T* p = partial + (long)(c0 + wid) * g;
+    T s[MD_WARPS];
+#pragma unroll
+    for (int w = 0; w < MD_WARPS; ++w) s[w] = T(0);
+    for (int q0 = 0; q0 < g; q0 += TPB)
+#pragma unroll
+      for (int w = 0; w < MD_WARPS; ++w) {
+        const int q = q0 + 32 * w + lane;
+        if (q < g) s[w] += ldcg_(p + q);
+      }
+    const T t8 = md_tree(s, lane);  // the sum of stride w in lane 4 * bit-reversed w
+    T t = T(0);
+#pragma unroll
+    for (int w = 0; w < MD_WARPS; ++w)
+      t += shfl_idx_any(t8, ((w >> 2) & 1) * 16 + ((w >> 1) & 1) * 8 + (w & 1) * 4);
+    if (lane == 0) out[c0 + wid] = t;
+  }
+  if (threadIdx.x == 0) *count = 0u;
+  return true;
+}
+
+// V^H w in one launch, a grid row of CTAs per group of CH columns.
+template <class T, int CH>
 __global__ void __launch_bounds__(TPB) mdot_kernel(long n, int k, const T* __restrict__ V, long ldv,
                                                    const T* __restrict__ w, unsigned char* __restrict__ buf,
                                                    T* __restrict__ out) {
   pdl_begin();
-  unsigned* count = reinterpret_cast<unsigned*>(buf);
-  T* partial = reinterpret_cast<T*>(buf + MD_HEAD);
-  const int g = gridDim.x;
-  const int c0 = blockIdx.y * MD_CH;
-  const int nc = min(MD_CH, k - c0);
-  T acc[MD_CH];
+  const int c0 = blockIdx.y * CH;
+  const int nc = min(CH, k - c0);
+  T acc[CH];
 #pragma unroll
-  for (int j = 0; j < MD_CH; ++j) acc[j] = T(0);
-  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
-    T wi = w[i];
+  for (int j = 0; j < CH; ++j) acc[j] = T(0);
+  // two rows' loads in flight at once, added in row order
+  const long step = (long)gridDim.x * TPB;
+  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += 2 * step) {
+    const bool two = i + step < n;
+    T v0[CH], v1[CH];
 #pragma unroll
-    for (int j = 0; j < MD_CH; ++j)
-      if (j < nc) acc[j] = fma_(cj(V[i + (long)(c0 + j) * ldv]), wi, acc[j]);
-  }
-  __shared__ T red[TPB / 32][MD_CH];
-  __shared__ bool last;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int j = 0; j < CH; ++j)
+      if (j < nc) {
+        v0[j] = V[i + (long)(c0 + j) * ldv];
+        v1[j] = two ? V[i + step + (long)(c0 + j) * ldv] : T(0);
+      }
+    const T w0 = w[i], w1 = two ? w[i + step] : T(0);
 #pragma unroll
-  for (int j = 0; j < MD_CH; ++j) {
-    T v = acc[j];
-    for (int o = 16; o > 0; o >>= 1) v += shfl_down(v, o);
-    if (lane == 0) red[wid][j] = v;
+    for (int j = 0; j < CH; ++j)
+      if (j < nc) {
+        acc[j] = fma_(cj(v0[j]), w0, acc[j]);
+        if (two) acc[j] = fma_(cj(v1[j]), w1, acc[j]);
+      }
   }
-  __syncthreads();
-  if (threadIdx.x < MD_CH) {
-    T v = T(0);
-    for (int q = 0; q < TPB / 32; ++q) v += red[q][threadIdx.x];
-    partial[(long)(c0 + threadIdx.x) * g + blockIdx.x] = v;
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(count, 1u) == (unsigned)(g * gridDim.y) - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  __shared__ T fin[TPB / 32];
-  for (int c = 0; c < k; ++c) {
-    T v = T(0);
-    for (int q = threadIdx.x; q < g; q += TPB) v += ldcg_(partial + (long)c * g + q);
-    for (int o = 16; o > 0; o >>= 1) v += shfl_down(v, o);
-    if (lane == 0) fin[wid] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      T t = T(0);
-      for (int q = 0; q < TPB / 32; ++q) t += fin[q];
-      out[c] = t;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *count = 0u;
+  md_finish<T, CH>(acc, nc, c0, buf, out);
 }
 template <class T> void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s) {
   if (k <= 0) return;
-  int g = md_grid(n);
-  dim3 grid(g, (k + MD_CH - 1) / MD_CH);
-  launch_k(mdot_kernel<T>, dim3(grid), dim3(TPB), 0, s, n, k, V, ldv, w, reinterpret_cast<unsigned char*>(partial),
-           out);
+  if (k > MD_CH * MD_GROUPS) throw std::runtime_error("mdot: too many columns");
+  unsigned char* buf = reinterpret_cast<unsigned char*>(partial);
+  const int g = md_grid(n);
+  if (k == 1)
+    launch_k(mdot_kernel<T, 1>, dim3(g), dim3(TPB), 0, s, n, k, V, ldv, w, buf, out);
+  else
+    launch_k(mdot_kernel<T, MD_CH>, dim3(g, (k + MD_CH - 1) / MD_CH), dim3(TPB), 0, s, n, k, V, ldv, w, buf, out);
   g_launches += 1;
 }
 
