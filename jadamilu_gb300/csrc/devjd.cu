@@ -377,8 +377,6 @@ correction:
       IFO = 0;
       const int MAXIT = ITCG;
       double GGK2 = GK * GK, RHO = 0, RHO1 = 0, TTK2 = 0, TTK2M = 0;
-      if (POSDEF) fill(N, H(0), Xc);
-      if (GEP) fill(N, H(0), BTv);
       int it = 0;
       bool fail = false;
       // RHO of iteration `it` is kept in device slot kScal + (it & 1), so the
@@ -386,34 +384,26 @@ correction:
       T* const scd = W->dsm + kScal;
       for (;;) {
         ++it;
-        if (device_ops && it > 1) {
-          // The same operations in the same order, with RHO, the projection
-          // coefficient, P^H Q, B-inner product and |R|^2 left on the
-          // device and read back together: one synchronisation per
-          // iteration.  The checks on RHO and P^H Q come after the read;
-          // a failed check leaves P, Q, Z and R modified where the plain
+        if (device_ops) {
+          // The same operations in the same order in six kernels beside the
+          // preconditioner, with RHO, the projection coefficient, the
+          // B-inner product, P^H Q and |R|^2 left on the device and read
+          // back together: one synchronisation per iteration.  The checks on
+          // RHO and P^H Q come after the read; a failed check leaves Q, Z
+          // and R (and P after the first iteration) modified where the plain
           // sequence stops earlier, and none of them is read after a failed
-          // inner solve (it > 1).
+          // inner solve.
           precond(R, Zv);
           S_.flagcg = true;
-          repgs(N, UU, BU, NEIG + 1, Zv, nullptr, EPSM, -1);
           T* rho_d = scd + (it & 1);
-          k::mdot<T>(N, 1, D(R), N, D(Zv), rho_d, W->dpart, S());
-          k::axpy_ratio_copy<T>(N, rho_d, scd + ((it - 1) & 1), D(P), D(Zv), D(P), S());
+          const T* rho0_d = it > 1 ? scd + ((it - 1) & 1) : nullptr;
+          k::mdot<T>(N, NEIG + 1, D(BU), N, D(Zv), W->dsm, W->dpart, S());
+          k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), rho_d, W->dpart, S());
+          k::cg_direction<T>(N, rho_d, rho0_d, POSDEF, D(P), D(Zv), S());
           AXPYALPHA = H(-ETA);
-          if (!GEP && matvec_shift) {
-            matvec_shift(P, Q, AXPYALPHA);
-          } else {
-            matvec(1, P, Q, Zv);
-            if (GEP) axpy(N, AXPYALPHA, Zv, Q);
-            else axpy(N, AXPYALPHA, P, Q);
-          }
-          if (GEP) k::mdot<T>(N, 1, D(BU), N, D(Q), scd + 4, W->dpart, S());
-          cgs_dev(N, BU, UU, 1, Q, scd + 2);
-          k::mdot<T>(N, 1, D(P), N, D(Q), scd + 3, W->dpart, S());
-          k::axpy_ratio<T>(N, rho_d, scd + 3, -1.0, D(Q), D(R), S());
-          k::mdot<T>(N, 1, D(R), N, D(R), scd + 5, W->dpart, S());
-          CK(cudaMemcpyAsync(W->hsm + kScal, scd, sizeof(T) * 6, cudaMemcpyDeviceToHost, S()));
+          matvec_dot(P, Q, Zv, AXPYALPHA, UU, BU, scd + 2);
+          k::gemv_dot<T>(N, 1, D(BU), N, scd + 2, D(Q), D(P), scd + 4, W->dpart, S());
+          k::cg_residual<T>(N, rho_d, scd + 4, D(Q), D(R), scd + 5, scd, 6, W->hsm + kScal, W->dpart, S());
           sync();
           const H* hs = reinterpret_cast<const H*>(W->hsm + kScal);
           RHO = hre(hs[it & 1]);
@@ -423,11 +413,11 @@ correction:
             break;
           }
           if (RHO == 0) { fail = true; break; }
-          if (GEP) AXPYALPHA = hs[4] / (NBU * NBU);
+          if (GEP) AXPYALPHA = hs[3] / (NBU * NBU);
           X[NP] = hs[2];
           ALPRHO = hre(X[NP]);
           ITER++;
-          alpha_cg = hre(hs[3]);
+          alpha_cg = hre(hs[4]);
           if ((POSDEF && alpha_cg <= 0) || alpha_cg == 0) { fail = true; break; }
           alpha_cg = RHO / alpha_cg;
           GK = std::sqrt(rl(W->hsm[kScal + 5]));
@@ -465,23 +455,16 @@ correction:
         axpy(N, H(-alpha_cg), Q, R);
         GK = nrm2(N, R);
         }
-        if (GEP) axpy(N, H(alpha_cg), Zv, BTv);
-        if (POSDEF) {
-          axpy(N, H(alpha_cg), P, Xc);
-        } else {
+        if (!POSDEF) {
           double GK2 = GK * GK;
           TTK2M = TTK2;
           TTK2 = GK2 / GGK2;
-          double CK2 = 1 / (1 + TTK2);
-          GGK2 = GGK2 * TTK2 * CK2;
-          if (it > 1) {
-            k::smooth<T>(N, todev(H(alpha_cg / TTK2M)), D(P), TTK2M * CK2, D(X2), D(Xc), S());
-          } else {
-            copy(N, P, X2);
-            scal(N, alpha_cg * CK2, X2);
-            copy(N, X2, Xc);
-          }
+          GGK2 = GGK2 * TTK2 * (1 / (1 + TTK2));
         }
+        const double CK2 = 1 / (1 + TTK2);
+        k::cg_iterate<T>(N, !POSDEF, it == 1, todev(H(POSDEF ? alpha_cg : alpha_cg / TTK2M)),
+                         it == 1 ? alpha_cg * CK2 : TTK2M * CK2, D(P), D(X2), D(Xc), todev(H(alpha_cg)), D(Zv),
+                         GEP ? D(BTv) : nullptr, S());
         if (FTFLG) IFO = (ISERCH == 2) ? -2 : -1;
         AXPYALPHA *= alpha_cg;
         ALPRHO *= alpha_cg;

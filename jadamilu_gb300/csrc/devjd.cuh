@@ -119,8 +119,9 @@ template <class T> struct DevJd {
   // which: 1 = A x (and B x for GEP), 3 = A x, 4 = B x; offsets into X
   std::function<void(int, long, long, long)> matvec;
   std::function<void(long, long)> precond;  // (rhs, sol)
-  // optional y = A x + a x in one pass (built-in matrix, no B)
-  std::function<void(long, long, H)> matvec_shift;
+  // built-in matrix: y = A x + a x (GEP: yb = B x, y = A x + a yb), out[0] = d0^H y
+  // and for GEP out[1] = d1^H y, in one kernel (offsets x, y, yb, d0, d1)
+  std::function<void(long, long, long, H, long, long, T*)> matvec_dot;
   std::function<void(int, int, int, double, double)> on_step;  // progress printer (may be empty)
   StopStateD<T> st;
   Lcg48d rng;
@@ -173,12 +174,6 @@ template <class T> struct DevJd {
     }
   }
   void axpy(long n, H a, long x, long y) { k::axpy<T>(n, todev(a), D(x), D(y), S()); }
-  // classical Gram-Schmidt of REPGS (gam < 0) with the coefficients left in
-  // device memory at cdev
-  void cgs_dev(long N, long V, long BV, long JV, long w, T* cdev) {
-    k::mdot<T>(N, (int)JV, D(BV), N, D(w), cdev, W->dpart, S());
-    k::gemv_dev<T>(N, (int)JV, T(-1), D(V), N, cdev, T(1), D(w), S());
-  }
   void scal(long n, double a, long x) { k::scal<T>(n, a, D(x), S()); }
   void copy(long n, long x, long y) {
     if (n > 0 && x != y) CK(cudaMemcpyAsync(D(y), D(x), sizeof(T) * n, cudaMemcpyDeviceToDevice, S()));

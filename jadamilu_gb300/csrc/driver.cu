@@ -935,9 +935,10 @@ template <class T> struct PjdRun {
     if (which == 1 || which == 3) k::spmv<T>(g.A, jd.D(x), jd.D(y), g.W.st);
     if ((which == 1 || which == 4) && gep) k::spmv<T>(g.Bm, jd.D(x), jd.D(by), g.W.st);
   }
-  void builtin_mv_shift(long x, long y, typename HostOf<T>::type a) {
+  void builtin_mv_dot(long x, long y, long yb, typename HostOf<T>::type a, long d0, long d1, T* out) {
     g.n_matvec++;
-    k::spmv_shift<T>(g.A, todev(a), jd.D(x), jd.D(y), g.W.st);
+    k::spmv_dot<T>(g.A, gep ? &g.Bm : nullptr, todev(a), jd.D(x), jd.D(y), jd.D(yb), jd.D(d0), jd.D(d1), out, g.W.dpart,
+                   g.W.st);
   }
   void precond(long rhs, long sol);
 };
@@ -1160,8 +1161,10 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
   else jd.matvec = [&R](int w, long x, long y, long by) { R.builtin_mv(w, x, y, by); };
   jd.precond = [&R](long r, long s) { R.precond(r, s); };
   jd.device_ops = !user_mv && g_opt.fuse_inner != 0;
-  if (jd.device_ops && !gep)
-    jd.matvec_shift = [&R](long x, long y, typename HostOf<T>::type a) { R.builtin_mv_shift(x, y, a); };
+  if (jd.device_ops)
+    jd.matvec_dot = [&R](long x, long y, long yb, typename HostOf<T>::type a, long d0, long d1, T* out) {
+      R.builtin_mv_dot(x, y, yb, a, d0, d1, out);
+    };
   if (R.P.pr >= 2)
     jd.on_step = [](int conv, int step, int k, double th, double v) {
       if (conv) std::printf("Step:%4d(%3d) ;  #MV:%7d ;  Rayl. quot.:%12.5E * converged\n\n", step, k, (int)v, th);

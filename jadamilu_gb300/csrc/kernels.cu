@@ -124,64 +124,11 @@ template <class T> void spmv(const SellMatrix<T>& A, const T* x, T* y, cudaStrea
   launch_k(spmv_sell_kernel<T>, dim3(nblk(A.n)), dim3(TPB), 0, s, A.n, A.sptr, A.col, A.val, x, y);
   COUNT_LAUNCH();
 }
-// y = A x + a x: the row sum, then the same fused multiply-add as axpy
-template <class T>
-__global__ void __launch_bounds__(TPB) spmv_shift_kernel(int n, const int64_t* __restrict__ sptr,
-                                                         const int* __restrict__ col, const T* __restrict__ val,
-                                                         T a, const T* __restrict__ x, T* __restrict__ y) {
-  pdl_launch();
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  int sl = r >> 5, lane = r & 31;
-  int64_t b = sptr[sl], e = sptr[sl + 1];
-  SellBatch<T> first;
-  sell_load(first, b + lane, e, col, val);
-  pdl_wait();
-  T acc = sell_use(first, x, T(0));
-  for (int64_t q = b + lane + kSellPre * 32; q < e; q += 32) acc = fma_(val[q], x[__ldg(col + q)], acc);
-  y[r] = fma_(a, x[r], acc);
-}
-template <class T> void spmv_shift(const SellMatrix<T>& A, T a, const T* x, T* y, cudaStream_t s) {
-  launch_k(spmv_shift_kernel<T>, dim3(nblk(A.n)), dim3(TPB), 0, s, A.n, A.sptr, A.col, A.val, a, x, y);
-  COUNT_LAUNCH();
-}
-
 // -------------------------------------------------------------- BLAS-1 ----
 template <class T> __global__ void axpy_kernel(long n, T a, const T* __restrict__ x, T* __restrict__ y) {
   pdl_begin();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     y[i] = fma_(a, x[i], y[i]);
-}
-// y += sign * (Re num / Re den) * x, the two scalars read from device memory
-// (results of earlier reductions on the same stream)
-template <class T>
-__global__ void axpy_ratio_kernel(long n, const T* num, const T* den, double sign, const T* __restrict__ x,
-                                  T* __restrict__ y) {
-  pdl_begin();
-  const T a = T(sign * (rl(*num) / rl(*den)));
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    y[i] = fma_(a, x[i], y[i]);
-}
-// y += (Re num / Re den) * x, then out = y (out may alias x)
-template <class T>
-__global__ void axpy_ratio_copy_kernel(long n, const T* num, const T* den, const T* x, T* __restrict__ y, T* out) {
-  pdl_begin();
-  const T a = T(1.0 * (rl(*num) / rl(*den)));
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const T t = fma_(a, x[i], y[i]);
-    y[i] = t;
-    out[i] = t;
-  }
-}
-// x2 = s (x2 + a p); xc = x2 + xc, as axpy, scal and axpy in sequence
-template <class T>
-__global__ void smooth_kernel(long n, T a, const T* __restrict__ p, double s, T* __restrict__ x2, T* __restrict__ xc) {
-  pdl_begin();
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const T t = s * fma_(a, p[i], x2[i]);
-    x2[i] = t;
-    xc[i] = fma_(T(1), t, xc[i]);
-  }
 }
 template <class T> __global__ void scal_kernel(long n, double a, T* x) {
   pdl_begin();
@@ -194,16 +141,6 @@ template <class T> __global__ void fill_kernel(long n, T v, T* x) {
 static inline int grid_1d(long n) { return (int)std::min<long>(nblk(n), 152L * 16); }
 template <class T> void axpy(long n, T a, const T* x, T* y, cudaStream_t s) {
   if (n > 0) { launch_k(axpy_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, a, x, y); COUNT_LAUNCH(); }
-}
-template <class T>
-void axpy_ratio(long n, const T* num, const T* den, double sign, const T* x, T* y, cudaStream_t s) {
-  if (n > 0) { launch_k(axpy_ratio_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, num, den, sign, x, y); COUNT_LAUNCH(); }
-}
-template <class T> void axpy_ratio_copy(long n, const T* num, const T* den, const T* x, T* y, T* out, cudaStream_t s) {
-  if (n > 0) { launch_k(axpy_ratio_copy_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, num, den, x, y, out); COUNT_LAUNCH(); }
-}
-template <class T> void smooth(long n, T a, const T* p, double sc, T* x2, T* xc, cudaStream_t s) {
-  if (n > 0) { launch_k(smooth_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, a, p, sc, x2, xc); COUNT_LAUNCH(); }
 }
 template <class T> void scal(long n, double a, T* x, cudaStream_t s) {
   if (n > 0) { launch_k(scal_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, a, x); COUNT_LAUNCH(); }
@@ -427,6 +364,193 @@ void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* yh, T beta,
   SmallVec<T> y;
   for (int c = 0; c < k; ++c) y.v[c] = yh[c];
   launch_k(jd_basis_gemv_val_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, k, alpha, V, ldv, y, beta, w);
+  COUNT_LAUNCH();
+}
+
+// ------------------------------------------- the inner iteration, fused ----
+// One CG / sQMR iteration outside the preconditioner is a chain of vector
+// updates with an inner product after each.  Every launch of the chain costs
+// about as much as its bytes up to n = 1e5, and an update's result is read
+// back by the inner product that follows, so each update kernel also
+// accumulates that product over the rows it writes, in the row order and with
+// the tail (md_finish) of mdot: the roundings are those of the separate
+// kernels.  Scalars stay in device memory (results of earlier kernels of the
+// chain); the last kernel puts them into pinned host memory itself.
+// Measured per solve, ten kernels and a copy before, six now (GB300): Anderson
+// 16^3 (n = 4096) 16 % less, Laplacian 20^3 51.6 -> 46.8 ms, tight-binding 64^3
+// (n = 262144, complex) 406 -> 389 ms.
+
+// w = w - V y (y in device memory), out[0] = x^H w (x = nullptr: w^H w)
+template <class T>
+__global__ void __launch_bounds__(TPB) gemv_dot_kernel(long n, int k, const T* __restrict__ V, long ldv, const T* y,
+                                                       T* w, const T* x, unsigned char* buf, T* out) {
+  pdl_begin();
+  __shared__ T ys[GMV_MAX];
+  if (threadIdx.x < k) ys[threadIdx.x] = y[threadIdx.x];
+  __syncthreads();
+  T dot[1] = {T(0)};
+  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
+    const T o = w[i], xi = x ? x[i] : T(0);
+    T acc = T(0);
+#pragma unroll 8
+    for (int c = 0; c < k; ++c) acc = fma_(V[i + (long)c * ldv], ys[c], acc);
+    const T r = fma_(T(-1), acc, o);
+    w[i] = r;
+    dot[0] = fma_(cj(x ? xi : r), r, dot[0]);
+  }
+  md_finish<T, 1>(dot, 1, 0, buf, out);
+}
+template <class T>
+void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s) {
+  if (k < 1 || k > GMV_MAX) throw std::runtime_error("projection against more than 64 vectors");
+  launch_k(gemv_dot_kernel<T>, dim3(md_grid(n)), dim3(TPB), 0, s, n, k, V, ldv, y, w, x,
+           reinterpret_cast<unsigned char*>(partial), out);
+  COUNT_LAUNCH();
+}
+
+// The search direction: z += (Re rho / Re rho0) p and p = z; the first
+// iteration (rho0 = nullptr) takes p = z, and leaves p alone when rho ends the
+// inner solve (zero, or not positive where the preconditioner should be), since
+// p is then its result.
+template <class T>
+__global__ void __launch_bounds__(TPB) cg_direction_kernel(long n, const T* rho, const T* rho0, bool posdef, T* p, T* z) {
+  pdl_begin();
+  if (!rho0) {
+    const double r = rl(*rho);
+    if (r == 0 || (posdef && r <= 0)) return;
+    for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) p[i] = z[i];
+    return;
+  }
+  const T a = T(rl(*rho) / rl(*rho0));
+  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
+    const T t = fma_(a, p[i], z[i]);
+    z[i] = t;
+    p[i] = t;
+  }
+}
+template <class T>
+void cg_direction(long n, const T* rho, const T* rho0, bool posdef, T* p, T* z, cudaStream_t s) {
+  launch_k(cg_direction_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, rho, rho0, posdef, p, z);
+  COUNT_LAUNCH();
+}
+
+// y = A x + a x, or with B: yb = B x, y = A x + a yb; out[c] = d[c]^H y for the
+// NC given columns.  Rows in mdot's order (a warp's 32 rows are one slice).
+template <class T> struct DotCols { const T* c[2]; };
+template <class T, bool GEP, int NC>
+__global__ void __launch_bounds__(TPB) spmv_dot_kernel(int n, const int64_t* __restrict__ sptr,
+                                                       const int* __restrict__ col, const T* __restrict__ val,
+                                                       const int64_t* __restrict__ bptr, const int* __restrict__ bcol,
+                                                       const T* __restrict__ bval, T a, const T* x, T* y, T* yb,
+                                                       DotCols<T> d, unsigned char* buf, T* out) {
+  pdl_launch();
+  T dot[NC];
+#pragma unroll
+  for (int j = 0; j < NC; ++j) dot[j] = T(0);
+  const int lane = threadIdx.x & 31;
+  bool waited = false;
+  for (int r = blockIdx.x * TPB + threadIdx.x; r < n; r += gridDim.x * TPB) {
+    const int sl = r >> 5;
+    const int64_t b = sptr[sl], e = sptr[sl + 1];
+    SellBatch<T> first, bfirst;
+    sell_load(first, b + lane, e, col, val);
+    int64_t b2 = 0, e2 = 0;
+    if (GEP) {
+      b2 = bptr[sl];
+      e2 = bptr[sl + 1];
+      sell_load(bfirst, b2 + lane, e2, bcol, bval);
+    }
+    if (!waited) {
+      pdl_wait();
+      waited = true;
+    }
+    T acc = sell_use(first, x, T(0));
+    for (int64_t q = b + lane + kSellPre * 32; q < e; q += 32) acc = fma_(val[q], x[__ldg(col + q)], acc);
+    T u;
+    if (GEP) {
+      T bc = sell_use(bfirst, x, T(0));
+      for (int64_t q = b2 + lane + kSellPre * 32; q < e2; q += 32) bc = fma_(bval[q], x[__ldg(bcol + q)], bc);
+      yb[r] = bc;
+      u = bc;
+    } else {
+      u = x[r];
+    }
+    const T t = fma_(a, u, acc);
+    y[r] = t;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) dot[j] = fma_(cj(d.c[j][r]), t, dot[j]);
+  }
+  if (!waited) pdl_wait();  // the reduction's buffer is the predecessor's too
+  md_finish<T, NC>(dot, NC, 0, buf, out);
+}
+template <class T>
+void spmv_dot(const SellMatrix<T>& A, const SellMatrix<T>* B, T a, const T* x, T* y, T* yb, const T* d0, const T* d1,
+              T* out, T* partial, cudaStream_t s) {
+  const dim3 g(md_grid(A.n)), t(TPB);
+  unsigned char* buf = reinterpret_cast<unsigned char*>(partial);
+  const DotCols<T> d{{d0, d1}};
+  const int64_t* bp = B ? B->sptr : nullptr;
+  const int* bc = B ? B->col : nullptr;
+  const T* bv = B ? B->val : nullptr;
+  auto go = [&](auto kern) { launch_k(kern, g, t, 0, s, A.n, A.sptr, A.col, A.val, bp, bc, bv, a, x, y, yb, d, buf, out); };
+  if (B) go(spmv_dot_kernel<T, true, 2>);
+  else go(spmv_dot_kernel<T, false, 1>);
+  COUNT_LAUNCH();
+}
+
+// r -= (Re num / Re den) q, out[0] = r^H r; the finishing CTA then copies the
+// iteration's nsc scalars (sc, out among them) to the host's pinned hsc.
+template <class T>
+__global__ void __launch_bounds__(TPB) cg_residual_kernel(long n, const T* num, const T* den, const T* __restrict__ q,
+                                                          T* __restrict__ r, unsigned char* buf, T* out, const T* sc,
+                                                          int nsc, T* hsc) {
+  pdl_begin();
+  const T a = T(-1.0 * (rl(*num) / rl(*den)));
+  T dot[1] = {T(0)};
+  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
+    const T t = fma_(a, q[i], r[i]);
+    r[i] = t;
+    dot[0] = fma_(cj(t), t, dot[0]);
+  }
+  if (!md_finish<T, 1>(dot, 1, 0, buf, out)) return;
+  __syncthreads();
+  if (threadIdx.x < nsc) hsc[threadIdx.x] = sc[threadIdx.x];
+}
+template <class T>
+void cg_residual(long n, const T* num, const T* den, const T* q, T* r, T* out, const T* sc, int nsc, T* hsc, T* partial,
+                 cudaStream_t s) {
+  launch_k(cg_residual_kernel<T>, dim3(md_grid(n)), dim3(TPB), 0, s, n, num, den, q, r,
+           reinterpret_cast<unsigned char*>(partial), out, sc, nsc, hsc);
+  COUNT_LAUNCH();
+}
+
+// The iterate: x += a p (CG), x2 = s (x2 + a p) and x += x2 (the smoothed form;
+// its first iteration: x2 = s p, x = x2); with B also bt += al bp.  The first
+// iteration's x and bt start from zero.
+template <class T, bool SMOOTH, bool FIRST>
+__global__ void __launch_bounds__(TPB) cg_iterate_kernel(long n, T a, double s, const T* __restrict__ p,
+                                                         T* __restrict__ x2, T* __restrict__ x, T al,
+                                                         const T* __restrict__ bp, T* __restrict__ bt) {
+  pdl_begin();
+  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
+    if (SMOOTH) {
+      const T t = FIRST ? s * p[i] : s * fma_(a, p[i], x2[i]);
+      x2[i] = t;
+      x[i] = FIRST ? t : fma_(T(1), t, x[i]);
+    } else {
+      x[i] = fma_(a, p[i], FIRST ? T(0) : x[i]);
+    }
+    if (bt) bt[i] = fma_(al, bp[i], FIRST ? T(0) : bt[i]);
+  }
+}
+template <class T>
+void cg_iterate(long n, bool smooth, bool first, T a, double sc, const T* p, T* x2, T* x, T al, const T* bp, T* bt,
+                cudaStream_t s) {
+  auto go = [&](auto kern) { launch_k(kern, dim3(grid_1d(n)), dim3(TPB), 0, s, n, a, sc, p, x2, x, al, bp, bt); };
+  if (smooth && first) go(cg_iterate_kernel<T, true, true>);
+  else if (smooth) go(cg_iterate_kernel<T, true, false>);
+  else if (first) go(cg_iterate_kernel<T, false, true>);
+  else go(cg_iterate_kernel<T, false, false>);
   COUNT_LAUNCH();
 }
 
@@ -1193,10 +1317,12 @@ template <class T, class S> void ildl_apply_graph(DevFactor<S>& F, bool spd, con
 #define JD_INST_T(T)                                                                               \
   template void spmv<T>(const SellMatrix<T>&, const T*, T*, cudaStream_t);                         \
   template void axpy<T>(long, T, const T*, T*, cudaStream_t);                                      \
-  template void axpy_ratio<T>(long, const T*, const T*, double, const T*, T*, cudaStream_t);        \
-  template void axpy_ratio_copy<T>(long, const T*, const T*, const T*, T*, T*, cudaStream_t);        \
-  template void smooth<T>(long, T, const T*, double, T*, T*, cudaStream_t);                         \
-  template void spmv_shift<T>(const SellMatrix<T>&, T, const T*, T*, cudaStream_t);                 \
+  template void gemv_dot<T>(long, int, const T*, long, const T*, T*, const T*, T*, T*, cudaStream_t); \
+  template void cg_direction<T>(long, const T*, const T*, bool, T*, T*, cudaStream_t);             \
+  template void spmv_dot<T>(const SellMatrix<T>&, const SellMatrix<T>*, T, const T*, T*, T*, const T*, const T*, \
+                            T*, T*, cudaStream_t);                                                \
+  template void cg_residual<T>(long, const T*, const T*, const T*, T*, T*, const T*, int, T*, T*, cudaStream_t); \
+  template void cg_iterate<T>(long, bool, bool, T, double, const T*, T*, T*, T, const T*, T*, cudaStream_t); \
   template void scal<T>(long, double, T*, cudaStream_t);                                           \
   template void fill<T>(long, T, T*, cudaStream_t);                                                \
   template void mdot<T>(long, int, const T*, long, const T*, T*, T*, cudaStream_t);                \

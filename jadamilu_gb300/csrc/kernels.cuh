@@ -109,15 +109,7 @@ void set_pdl(bool on);
 void add_launches(long long n);
 
 template <class T> void spmv(const SellMatrix<T>& A, const T* x, T* y, cudaStream_t s);
-// y = A x + a x (the shifted operator of the correction equation)
-template <class T> void spmv_shift(const SellMatrix<T>& A, T a, const T* x, T* y, cudaStream_t s);
 template <class T> void axpy(long n, T a, const T* x, T* y, cudaStream_t s);
-// y += sign * (Re *num / Re *den) * x with num and den in device memory
-template <class T> void axpy_ratio(long n, const T* num, const T* den, double sign, const T* x, T* y, cudaStream_t s);
-// y += (Re *num / Re *den) * x; out = y (out may alias x)
-template <class T> void axpy_ratio_copy(long n, const T* num, const T* den, const T* x, T* y, T* out, cudaStream_t s);
-// x2 = s (x2 + a p); xc += x2 (axpy, scal, axpy with the same roundings)
-template <class T> void smooth(long n, T a, const T* p, double sc, T* x2, T* xc, cudaStream_t s);
 template <class T> void scal(long n, double a, T* x, cudaStream_t s);
 template <class T> void fill(long n, T v, T* x, cudaStream_t s);
 // out[c] = V(:,c)^H w for c < k (deterministic two-pass reduction); partial
@@ -127,6 +119,26 @@ template <class T> void mdot(long n, int k, const T* V, long ldv, const T* w, T*
 // w = beta*w + alpha*V*y, y (k <= 64 entries) in device memory or by value
 template <class T> void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, T* w, cudaStream_t s);
 template <class T> void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* y_host, T beta, T* w, cudaStream_t s);
+// The kernels of one fused CG / sQMR iteration (kernels.cu); partial as for mdot.
+// w -= V y (y in device memory, 1 <= k <= 64), *out = x^H w (x null: w^H w)
+template <class T>
+void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s);
+// z += (Re *rho / Re *rho0) p, p = z; rho0 null: p = z unless *rho ends the solve
+template <class T>
+void cg_direction(long n, const T* rho, const T* rho0, bool posdef, T* p, T* z, cudaStream_t s);
+// y = A x + a x, out[0] = d0^H y; with B: yb = B x, y = A x + a yb, out[0..1] = d0^H y, d1^H y
+template <class T>
+void spmv_dot(const SellMatrix<T>& A, const SellMatrix<T>* B, T a, const T* x, T* y, T* yb, const T* d0, const T* d1,
+              T* out, T* partial, cudaStream_t s);
+// r -= (Re *num / Re *den) q, *out = r^H r, then hsc[0..nsc) = sc[0..nsc) (hsc: pinned host memory)
+template <class T>
+void cg_residual(long n, const T* num, const T* den, const T* q, T* r, T* out, const T* sc, int nsc, T* hsc, T* partial,
+                 cudaStream_t s);
+// smooth: x2 = sc (x2 + a p), x += x2 (first: x2 = sc p, x = x2); else x += a p (first: from zero); bt, when given,
+// += al bp (first: from zero)
+template <class T>
+void cg_iterate(long n, bool smooth, bool first, T a, double sc, const T* p, T* x2, T* x, T al, const T* bp, T* bt,
+                cudaStream_t s);
 // out(:,c) = V * Q(:,c), c < keep, Q K x K column-major (host values)
 template <class T> void rmult(long n, int K, int keep, const T* V, long ldv, const T* Q_host, T* out, cudaStream_t s);
 // sol = d .* rhs (diagonal preconditioner, d real)
