@@ -148,7 +148,7 @@ void DevJd<T>::run(long N, double* EIGS, double* RES, int LXi, int& NEIG, double
   double ETA1 = RINF, ETA0 = SIGMA, DELTA1 = RINF, NREIG = RINF, RESID = RINF, RNDIND = 0, DELTAO = 0;
   if (ISERCH == 0) ETA0 = RINF;
   const long MIDSPACE = (MOD + 1) / 2;
-  bool INITFLG = false, UKNOWN = false, CONV = false;
+  bool INITFLG = false, UKNOWN = false, CONV = false, ritz_late = false;
   double THETA = 0, THETA2 = 0, THMT = 0, NBU = 1, NREIGP = 0, TRS = 0, ETA = 0, SCLR1 = 0, SCLR2 = 0, ALPRHO = 0,
          GK = 0;
   H AXPYALPHA = H(0), AXPYBETA = H(0);
@@ -236,17 +236,23 @@ main_loop:
       SCLR1 = jdd::nrm2(J, X + YY);
       jdd::rscal(J, 1 / SCLR1, X + YY);
     }
-    gemvn(N, (int)J, H(1), VV, N, X + YY, H(0), UU);
-    gemvn(N, (int)J, H(1), WW, N, X + YY, H(0), REIG);
-    if (GEP) gemvn(N, (int)J, H(1), BV, N, X + YY, H(0), BU);
+    // the Ritz vector and its residual in one kernel once THMT is known: for
+    // GEP's harmonic extraction it needs |B u| first
+    ritz_late = !(GEP && ISERCH == 2);
+    if (!ritz_late) {
+      gemvn(N, (int)J, H(1), VV, N, X + YY, H(0), UU);
+      gemvn(N, (int)J, H(1), WW, N, X + YY, H(0), REIG);
+      gemvn(N, (int)J, H(1), BV, N, X + YY, H(0), BU);
+    }
   } else {
+    ritz_late = false;
     X[YY] = H(1);
     jdd::fillv(J - 1, H(0), X + YY + 1);
     copy(N, VV, UU);
     copy(N, WW, REIG);
     if (GEP) copy(N, BV, BU);
   }
-  if (GEP) NBU = nrm2(N, BU);
+  if (GEP && !ritz_late) NBU = nrm2(N, BU);
   if (ISERCH == 2) {
     if (GEP) {
       jdd::gemv_n(J, J, H(1), X + MM, MOD, X + YY, H(0), X + WL);
@@ -260,9 +266,19 @@ main_loop:
     THMT = THETA;
     ETA0 = std::min(ETA0, THETA);
   }
-  axpy(N, H(-THMT), BU, REIG);
   NREIGP = NREIG;
-  NREIG = nrm2(N, REIG);
+  if (ritz_late) {
+    T y[32];
+    for (long c = 0; c < J; ++c) y[c] = todev(X[YY + c]);
+    k::ritz<T>(N, (int)J, D(VV), D(WW), GEP ? D(BV) : nullptr, N, y, todev(H(-THMT)), D(UU), D(REIG),
+               GEP ? D(BU) : nullptr, W->hsm, W->dpart, S());
+    sync();
+    NREIG = std::sqrt(rl(W->hsm[0]));
+    if (GEP) NBU = std::sqrt(rl(W->hsm[1]));
+  } else {
+    axpy(N, H(-THMT), BU, REIG);
+    NREIG = nrm2(N, REIG);
+  }
   if (GEP) NREIG /= NBU;
   if (neweig) { S_.rinit = NREIG; neweig = false; }
   if (std::fabs(NREIG / NREIGP - 1) < 0.01) istag++;
@@ -357,7 +373,6 @@ correction:
     if (NREIG < std::fabs(DELTA1) && std::fabs(DELTA1 / DELTAO - 1) < 0.1) ETA = THETA;
   }
   repgs(N, BU, UU, NEIG + 1, REIG, X + WL, EPSM, -1);
-  RNDIND = habs(X[WL + NEIG]) / (NREIG * EPSMSR);
   RESID = NREIG;
   {
     const long XCG = VV + J * N;
@@ -369,7 +384,7 @@ correction:
       S_.shift1 = THETA;
       GAP = (J > 1) ? THETA2 - THETA : 0;
     }
-    if (GEP) AXPYBETA = dot(N, BU, REIG) / (NBU * NBU);
+    if (GEP) k::mdot<T>(N, 1, D(BU), N, D(REIG), W->hsm + kLate, W->dpart, S());
     const long R = WCG, Zv = WCG + N, P = WCG + 2 * N, Q = WCG + 3 * N, X2 = XCG2, BTv = BT, Xc = XCG;
     bool FTFLG = true;
     {
@@ -424,9 +439,9 @@ correction:
         } else {
         precond(R, Zv);
         S_.flagcg = true;
-        repgs(N, UU, BU, NEIG + 1, Zv, nullptr, EPSM, -1);
-        k::mdot<T>(N, 1, D(R), N, D(Zv), scd + (it & 1), W->dpart, S());
-        CK(cudaMemcpyAsync(W->hsm + kScal, scd + (it & 1), sizeof(T), cudaMemcpyDeviceToHost, S()));
+        if (NEIG + 1 > 64) throw std::runtime_error("projection against more than 64 vectors");
+        k::mdot<T>(N, NEIG + 1, D(BU), N, D(Zv), W->dsm, W->dpart, S());
+        k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), W->hsm + kScal, W->dpart, S());
         sync();
         RHO = hre(reinterpret_cast<const H*>(W->hsm + kScal)[0]);
         if (POSDEF && RHO <= 0) {
@@ -446,10 +461,13 @@ correction:
         if (GEP) axpy(N, AXPYALPHA, Zv, Q);
         else axpy(N, AXPYALPHA, P, Q);
         if (GEP) AXPYALPHA = dot(N, BU, Q) / (NBU * NBU);
-        repgs(N, BU, UU, 1, Q, X + NP, EPSM, -1);
+        k::mdot<T>(N, 1, D(UU), N, D(Q), W->dsm, W->dpart, S());
+        k::gemv_dot<T>(N, 1, D(BU), N, W->dsm, D(Q), D(P), W->dsm + 1, W->dpart, S(), W->dsm, 2, W->hsm + kScal);
+        sync();
+        X[NP] = reinterpret_cast<const H*>(W->hsm)[kScal];
         ALPRHO = hre(X[NP]);
         ITER++;
-        alpha_cg = hre(dot(N, P, Q));
+        alpha_cg = hre(reinterpret_cast<const H*>(W->hsm)[kScal + 1]);
         if ((POSDEF && alpha_cg <= 0) || alpha_cg == 0) { fail = true; break; }
         alpha_cg = RHO / alpha_cg;
         axpy(N, H(-alpha_cg), Q, R);
@@ -466,6 +484,7 @@ correction:
                          it == 1 ? alpha_cg * CK2 : TTK2M * CK2, D(P), D(X2), D(Xc), todev(H(alpha_cg)), D(Zv),
                          GEP ? D(BTv) : nullptr, S());
         if (FTFLG) IFO = (ISERCH == 2) ? -2 : -1;
+        if (FTFLG && GEP) AXPYBETA = reinterpret_cast<const H*>(W->hsm)[kLate] / (NBU * NBU);
         AXPYALPHA *= alpha_cg;
         ALPRHO *= alpha_cg;
         stoptest(N, Xc, BTv, BU, TOL, RESID, NBU, ALPRHO, GK, AXPYALPHA, AXPYBETA, THETA, ETA, IFO, TRS, GEP);
@@ -480,6 +499,7 @@ correction:
         if (it == 1) copy(N, P, Xc);
       }
     }
+    RNDIND = habs(repgs_coef(NEIG)) / (NREIG * EPSMSR);  // every inner iteration has synchronised
     if (ISERCH != 2 && ETA <= ETA0 && NEIG > 0 && IFO == 2) ETA0 = std::min(ETA1, ETA0);
     CONV = false;
     S_.flagcg = false;
@@ -523,10 +543,12 @@ correction:
       gemvc(N, (int)J + 1, WW, N, NDX3, X + MM + J * MOD);
       gemvc(N, (int)J, BV, N, NDX2, t1.data());
       for (long r = 0; r < J; ++r) X[MM + J + r * MOD] = jdd::cj(t1[r]);
+      gemvc(N, (int)J + 1, WW, N, NDX2, X + NN + J * MOD);
+    } else if (ISERCH == 2) {
+      gemvc2(N, (int)J + 1, VV, WW, N, NDX2, X + MM + J * MOD, X + NN + J * MOD);
     } else {
       gemvc(N, (int)J + 1, VV, N, NDX2, X + MM + J * MOD);
     }
-    if (ISERCH == 2) gemvc(N, (int)J + 1, WW, N, NDX2, X + NN + J * MOD);
     J++;
     UKNOWN = false;
     if (!CONV) goto main_loop;

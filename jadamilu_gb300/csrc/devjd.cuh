@@ -132,22 +132,24 @@ template <class T> struct DevJd {
   // round trip inside matvec/precond): the inner iteration may then keep its
   // scalars on the device and read them back once per iteration.
   bool device_ops = false;
-  static constexpr int kScal = 500;  // dsm slots of the inner-iteration scalars
+  static constexpr int kScal = 500;  // dsm / hsm slots of the inner-iteration scalars
+  static constexpr int kCoef = 320;  // hsm slots of a projection's coefficients (64), read at a later synchronisation
+  static constexpr int kLate = 400;  // hsm slot of an inner product read at a later synchronisation
 
   T* D(long off) { return W->dX + off; }
   cudaStream_t S() { return W->st; }
   void sync() { CK(cudaStreamSynchronize(S())); }
 
   // ---- device primitives on X offsets ----
+  // (a reduction whose result only the host needs writes it straight into
+  // the pinned mirror)
   double nrm2(long n, long x) {
-    k::mdot<T>(n, 1, D(x), n, D(x), W->dsm, W->dpart, S());
-    CK(cudaMemcpyAsync(W->hsm, W->dsm, sizeof(T), cudaMemcpyDeviceToHost, S()));
+    k::mdot<T>(n, 1, D(x), n, D(x), W->hsm, W->dpart, S());
     sync();
     return std::sqrt(rl(W->hsm[0]));
   }
   H dot(long n, long x, long y) {
-    k::mdot<T>(n, 1, D(x), n, D(y), W->dsm, W->dpart, S());
-    CK(cudaMemcpyAsync(W->hsm, W->dsm, sizeof(T), cudaMemcpyDeviceToHost, S()));
+    k::mdot<T>(n, 1, D(x), n, D(y), W->hsm, W->dpart, S());
     sync();
     return reinterpret_cast<H*>(W->hsm)[0];
   }
@@ -156,10 +158,25 @@ template <class T> struct DevJd {
     if (kc <= 0) return;
     for (int c0 = 0; c0 < kc; c0 += 128) {
       int kk = std::min(128, kc - c0);
-      k::mdot<T>(n, kk, D(V + (long)c0 * ldv), ldv, D(w), W->dsm, W->dpart, S());
-      CK(cudaMemcpyAsync(W->hsm, W->dsm, sizeof(T) * kk, cudaMemcpyDeviceToHost, S()));
+      k::mdot<T>(n, kk, D(V + (long)c0 * ldv), ldv, D(w), W->hsm, W->dpart, S());
       sync();
       for (int c = 0; c < kk; ++c) out_host[c0 + c] = reinterpret_cast<H*>(W->hsm)[c];
+    }
+  }
+  // two of them with the same vector, read together (at most 64 columns each)
+  void gemvc2(long n, int kc, long V, long V2, long ldv, long w, H* out, H* out2) {
+    if (kc > 64) {
+      gemvc(n, kc, V, ldv, w, out);
+      gemvc(n, kc, V2, ldv, w, out2);
+      return;
+    }
+    k::mdot<T>(n, kc, D(V), ldv, D(w), W->hsm, W->dpart, S());
+    k::mdot<T>(n, kc, D(V2), ldv, D(w), W->hsm + 64, W->dpart, S());
+    sync();
+    const H* h = reinterpret_cast<const H*>(W->hsm);
+    for (int c = 0; c < kc; ++c) {
+      out[c] = h[c];
+      out2[c] = h[64 + c];
     }
   }
   // X(w) = beta X(w) + alpha X(V) y, y on the host
@@ -185,27 +202,43 @@ template <class T> struct DevJd {
     bool nrnd = true;
     if (JV <= 0) return;
     if (gam < 0) {
-      // classical Gram-Schmidt, coefficients stay on the device
+      // classical Gram-Schmidt, coefficients stay on the device; y, when
+      // given, is filled after the next synchronisation by repgs_coef
       if (JV > 64) throw std::runtime_error("projection against more than 64 vectors");
       k::mdot<T>(N, (int)JV, D(BV), N, D(w), W->dsm, W->dpart, S());
-      k::gemv_dev<T>(N, (int)JV, T(-1), D(V), N, W->dsm, T(1), D(w), S());
-      if (y) {
-        CK(cudaMemcpyAsync(W->hsm, W->dsm, sizeof(T) * JV, cudaMemcpyDeviceToHost, S()));
-        sync();
-        for (long c = 0; c < JV; ++c) y[c] = reinterpret_cast<H*>(W->hsm)[c];
-      }
+      k::gemv_dev<T>(N, (int)JV, T(-1), D(V), N, W->dsm, T(1), D(w), S(), y ? W->hsm + kCoef : nullptr);
       return;
     }
+    // up to 63 columns: a pass leaves its coefficients on the device between
+    // the inner products and the update, which also gives the new norm (and
+    // the first pass takes the old norm as one more column), and is read back
+    // once
+    const bool one_read = JV < 64;
     for (;;) {
-      double nrn = nrm2(N, w), nr = epsm * nrn, nro;
+      double nrn = one_read ? 0.0 : nrm2(N, w), nr = epsm * nrn, nro;
       if (nrnd)
         for (long c = 0; c < JV; ++c) y[c] = H(0);
-      bool small = false;
+      bool small = false, first = true;
       do {
         nro = nrn;
-        gemvc(N, (int)JV, BV, N, w, y + JV);
-        gemvn(N, (int)JV, H(-1), V, N, y + JV, H(1), w);
-        nrn = nrm2(N, w);
+        if (one_read) {
+          k::mdot<T>(N, (int)JV + first, D(BV), N, D(w), W->dsm, W->dpart, S(), first ? D(w) : nullptr);
+          k::gemv_dot<T>(N, (int)JV, D(V), N, W->dsm, D(w), nullptr, W->dsm + JV + 1, W->dpart, S(), W->dsm,
+                         (int)JV + 2, W->hsm);
+          sync();
+          const H* h = reinterpret_cast<const H*>(W->hsm);
+          for (long c = 0; c < JV; ++c) y[JV + c] = h[c];
+          if (first) {
+            nro = std::sqrt(rl(W->hsm[JV]));
+            nr = epsm * nro;
+          }
+          nrn = std::sqrt(rl(W->hsm[JV + 1]));
+          first = false;
+        } else {
+          gemvc(N, (int)JV, BV, N, w, y + JV);
+          gemvn(N, (int)JV, H(-1), V, N, y + JV, H(1), w);
+          nrn = nrm2(N, w);
+        }
         if (nrnd)
           for (long c = 0; c < JV; ++c) y[c] += y[JV + c];
         if (nrn <= nr) { small = true; break; }
@@ -227,6 +260,9 @@ template <class T> struct DevJd {
       return;
     }
   }
+
+  // coefficient c of the last projection with gam < 0 (valid after a synchronisation)
+  H repgs_coef(long c) const { return reinterpret_cast<const H*>(W->hsm)[kCoef + c]; }
 
   // SORTEV on host arrays (small) or device columns (eigenvectors)
   void sort_index_key(long J, const double* eigs, int it, double sigma, std::vector<long>& iw) {

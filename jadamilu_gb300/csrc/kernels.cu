@@ -269,13 +269,17 @@ __device__ __forceinline__ bool md_finish(T (&acc)[CH], int nc, int c0, unsigned
 }
 
 // V^H w in one launch, a grid row of CTAs per group of CH columns.
+// xcol, when given, is column k - 1 (a vector that does not follow V's others).
 template <class T, int CH>
 __global__ void __launch_bounds__(TPB) mdot_kernel(long n, int k, const T* __restrict__ V, long ldv,
-                                                   const T* __restrict__ w, unsigned char* __restrict__ buf,
-                                                   T* __restrict__ out) {
+                                                   const T* __restrict__ w, const T* __restrict__ xcol,
+                                                   unsigned char* __restrict__ buf, T* __restrict__ out) {
   pdl_begin();
   const int c0 = blockIdx.y * CH;
   const int nc = min(CH, k - c0);
+  const T* cp[CH];
+#pragma unroll
+  for (int j = 0; j < CH; ++j) cp[j] = xcol && c0 + j == k - 1 ? xcol : V + (long)(c0 + j) * ldv;
   T acc[CH];
 #pragma unroll
   for (int j = 0; j < CH; ++j) acc[j] = T(0);
@@ -287,8 +291,8 @@ __global__ void __launch_bounds__(TPB) mdot_kernel(long n, int k, const T* __res
 #pragma unroll
     for (int j = 0; j < CH; ++j)
       if (j < nc) {
-        v0[j] = V[i + (long)(c0 + j) * ldv];
-        v1[j] = two ? V[i + step + (long)(c0 + j) * ldv] : T(0);
+        v0[j] = cp[j][i];
+        v1[j] = two ? cp[j][i + step] : T(0);
       }
     const T w0 = w[i], w1 = two ? w[i + step] : T(0);
 #pragma unroll
@@ -300,15 +304,16 @@ __global__ void __launch_bounds__(TPB) mdot_kernel(long n, int k, const T* __res
   }
   md_finish<T, CH>(acc, nc, c0, buf, out);
 }
-template <class T> void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s) {
+template <class T>
+void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s, const T* xcol) {
   if (k <= 0) return;
   if (k > MD_CH * MD_GROUPS) throw std::runtime_error("mdot: too many columns");
   unsigned char* buf = reinterpret_cast<unsigned char*>(partial);
   const int g = md_grid(n);
   if (k == 1)
-    launch_k(mdot_kernel<T, 1>, dim3(g), dim3(TPB), 0, s, n, k, V, ldv, w, buf, out);
+    launch_k(mdot_kernel<T, 1>, dim3(g), dim3(TPB), 0, s, n, k, V, ldv, w, xcol, buf, out);
   else
-    launch_k(mdot_kernel<T, MD_CH>, dim3(g, (k + MD_CH - 1) / MD_CH), dim3(TPB), 0, s, n, k, V, ldv, w, buf, out);
+    launch_k(mdot_kernel<T, MD_CH>, dim3(g, (k + MD_CH - 1) / MD_CH), dim3(TPB), 0, s, n, k, V, ldv, w, xcol, buf, out);
   g_launches += 1;
 }
 
@@ -318,10 +323,14 @@ template <class T> struct SmallVec { T v[GMV_MAX]; };
 
 template <class T>
 __global__ void __launch_bounds__(TPB) jd_basis_gemv_dev_kernel(long n, int k, T alpha, const T* __restrict__ V, long ldv,
-                                                       const T* __restrict__ y, T beta, T* __restrict__ w) {
+                                                       const T* __restrict__ y, T beta, T* __restrict__ w,
+                                                       T* __restrict__ hy) {
   pdl_begin();
   __shared__ T ys[GMV_MAX];
-  if (threadIdx.x < k) ys[threadIdx.x] = y[threadIdx.x];
+  if (threadIdx.x < k) {
+    ys[threadIdx.x] = y[threadIdx.x];
+    if (hy && blockIdx.x == 0) hy[threadIdx.x] = ys[threadIdx.x];
+  }
   __syncthreads();
   for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
     T acc = T(0);
@@ -342,7 +351,7 @@ __global__ void __launch_bounds__(TPB) jd_basis_gemv_val_kernel(long n, int k, T
   }
 }
 template <class T>
-void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, T* w, cudaStream_t s) {
+void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, T* w, cudaStream_t s, T* hy) {
   if (k > GMV_MAX) throw std::runtime_error("gemv_dev: too many columns");
   if (k <= 0) {
     if (!(beta == T(1))) {
@@ -351,7 +360,7 @@ void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, 
     }
     return;
   }
-  launch_k(jd_basis_gemv_dev_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, k, alpha, V, ldv, y, beta, w);
+  launch_k(jd_basis_gemv_dev_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, k, alpha, V, ldv, y, beta, w, hy);
   COUNT_LAUNCH();
 }
 template <class T>
@@ -380,31 +389,46 @@ void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* yh, T beta,
 // 16^3 (n = 4096) 16 % less, Laplacian 20^3 51.6 -> 46.8 ms, tight-binding 64^3
 // (n = 262144, complex) 406 -> 389 ms.
 
-// w = w - V y (y in device memory), out[0] = x^H w (x = nullptr: w^H w)
+// w = w - V y (y in device memory), out[0] = x^H w (x = nullptr: w^H w); then,
+// with nsc > 0, the nsc scalars from sc on go to the host's pinned hsc.
 template <class T>
 __global__ void __launch_bounds__(TPB) gemv_dot_kernel(long n, int k, const T* __restrict__ V, long ldv, const T* y,
-                                                       T* w, const T* x, unsigned char* buf, T* out) {
+                                                       T* w, const T* x, unsigned char* buf, T* out, const T* sc,
+                                                       int nsc, T* hsc) {
   pdl_begin();
   __shared__ T ys[GMV_MAX];
   if (threadIdx.x < k) ys[threadIdx.x] = y[threadIdx.x];
   __syncthreads();
   T dot[1] = {T(0)};
-  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
-    const T o = w[i], xi = x ? x[i] : T(0);
-    T acc = T(0);
-#pragma unroll 8
-    for (int c = 0; c < k; ++c) acc = fma_(V[i + (long)c * ldv], ys[c], acc);
-    const T r = fma_(T(-1), acc, o);
-    w[i] = r;
-    dot[0] = fma_(cj(x ? xi : r), r, dot[0]);
+  const long step = (long)gridDim.x * TPB;
+  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += 2 * step) {  // two rows at once, as mdot
+    const bool two = i + step < n;
+    const long i1 = two ? i + step : i;
+    const T o0 = w[i], o1 = w[i1], x0 = x ? x[i] : T(0), x1 = x ? x[i1] : T(0);
+    T a0 = T(0), a1 = T(0);
+#pragma unroll 4
+    for (int c = 0; c < k; ++c) {
+      a0 = fma_(V[i + (long)c * ldv], ys[c], a0);
+      a1 = fma_(V[i1 + (long)c * ldv], ys[c], a1);
+    }
+    const T r0 = fma_(T(-1), a0, o0), r1 = fma_(T(-1), a1, o1);
+    w[i] = r0;
+    dot[0] = fma_(cj(x ? x0 : r0), r0, dot[0]);
+    if (two) {
+      w[i1] = r1;
+      dot[0] = fma_(cj(x ? x1 : r1), r1, dot[0]);
+    }
   }
-  md_finish<T, 1>(dot, 1, 0, buf, out);
+  if (!md_finish<T, 1>(dot, 1, 0, buf, out)) return;
+  __syncthreads();
+  if (threadIdx.x < nsc) hsc[threadIdx.x] = sc[threadIdx.x];
 }
 template <class T>
-void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s) {
+void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s,
+              const T* sc, int nsc, T* hsc) {
   if (k < 1 || k > GMV_MAX) throw std::runtime_error("projection against more than 64 vectors");
   launch_k(gemv_dot_kernel<T>, dim3(md_grid(n)), dim3(TPB), 0, s, n, k, V, ldv, y, w, x,
-           reinterpret_cast<unsigned char*>(partial), out);
+           reinterpret_cast<unsigned char*>(partial), out, sc, nsc, hsc);
   COUNT_LAUNCH();
 }
 
@@ -551,6 +575,65 @@ void cg_iterate(long n, bool smooth, bool first, T a, double sc, const T* p, T* 
   else if (smooth) go(cg_iterate_kernel<T, true, false>);
   else if (first) go(cg_iterate_kernel<T, false, true>);
   else go(cg_iterate_kernel<T, false, false>);
+  COUNT_LAUNCH();
+}
+
+// The Ritz vector and its residual: u = V y, r = W y + a bu (bu = u, or B y
+// for the generalized problem), out[0] = r^H r (and out[1] = bu^H bu), y by
+// value; one pass over the bases instead of one kernel per vector and one for
+// the norm, with their roundings.
+template <class T, bool GEP>
+__global__ void __launch_bounds__(TPB) ritz_kernel(long n, int k, const T* __restrict__ V, const T* __restrict__ Wv,
+                                                   const T* __restrict__ B, long ld, SmallVec<T> y, T a,
+                                                   T* __restrict__ u, T* __restrict__ r, T* __restrict__ bu,
+                                                   unsigned char* buf, T* out) {
+  pdl_begin();
+  T dot[GEP ? 2 : 1];
+  dot[0] = T(0);
+  if (GEP) dot[GEP] = T(0);
+  const long step = (long)gridDim.x * TPB;
+  for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += 2 * step) {  // two rows at once, as mdot
+    const long at[2] = {i, i + step < n ? i + step : i};
+    T su[2], sr[2], sb[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) su[q] = sr[q] = sb[q] = T(0);
+#pragma unroll 2
+    for (int c = 0; c < k; ++c)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        su[q] = fma_(V[at[q] + (long)c * ld], y.v[c], su[q]);
+        sr[q] = fma_(Wv[at[q] + (long)c * ld], y.v[c], sr[q]);
+        if (GEP) sb[q] = fma_(B[at[q] + (long)c * ld], y.v[c], sb[q]);
+      }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (q == 1 && i + step >= n) break;
+      T ub = fma_(T(1), su[q], T(0));
+      u[at[q]] = ub;
+      if (GEP) {
+        ub = fma_(T(1), sb[q], T(0));
+        bu[at[q]] = ub;
+        dot[GEP] = fma_(cj(ub), ub, dot[GEP]);
+      }
+      const T t = fma_(a, ub, fma_(T(1), sr[q], T(0)));
+      r[at[q]] = t;
+      dot[0] = fma_(cj(t), t, dot[0]);
+    }
+  }
+  md_finish<T, GEP ? 2 : 1>(dot, GEP ? 2 : 1, 0, buf, out);
+}
+template <class T>
+void ritz(long n, int k, const T* V, const T* Wv, const T* B, long ld, const T* yh, T a, T* u, T* r, T* bu, T* out,
+          T* partial, cudaStream_t s) {
+  if (k < 1 || k > GMV_MAX) throw std::runtime_error("ritz: bad column count");
+  SmallVec<T> y;
+  for (int c = 0; c < k; ++c) y.v[c] = yh[c];
+  auto go = [&](auto kern) {
+    launch_k(kern, dim3(md_grid(n)), dim3(TPB), 0, s, n, k, V, Wv, B, ld, y, a, u, r, bu,
+             reinterpret_cast<unsigned char*>(partial), out);
+  };
+  if (B) go(ritz_kernel<T, true>);
+  else go(ritz_kernel<T, false>);
   COUNT_LAUNCH();
 }
 
@@ -1317,7 +1400,8 @@ template <class T, class S> void ildl_apply_graph(DevFactor<S>& F, bool spd, con
 #define JD_INST_T(T)                                                                               \
   template void spmv<T>(const SellMatrix<T>&, const T*, T*, cudaStream_t);                         \
   template void axpy<T>(long, T, const T*, T*, cudaStream_t);                                      \
-  template void gemv_dot<T>(long, int, const T*, long, const T*, T*, const T*, T*, T*, cudaStream_t); \
+  template void gemv_dot<T>(long, int, const T*, long, const T*, T*, const T*, T*, T*, cudaStream_t, const T*, int, \
+                            T*);                                                                  \
   template void cg_direction<T>(long, const T*, const T*, bool, T*, T*, cudaStream_t);             \
   template void spmv_dot<T>(const SellMatrix<T>&, const SellMatrix<T>*, T, const T*, T*, T*, const T*, const T*, \
                             T*, T*, cudaStream_t);                                                \
@@ -1325,8 +1409,9 @@ template <class T, class S> void ildl_apply_graph(DevFactor<S>& F, bool spd, con
   template void cg_iterate<T>(long, bool, bool, T, double, const T*, T*, T*, T, const T*, T*, cudaStream_t); \
   template void scal<T>(long, double, T*, cudaStream_t);                                           \
   template void fill<T>(long, T, T*, cudaStream_t);                                                \
-  template void mdot<T>(long, int, const T*, long, const T*, T*, T*, cudaStream_t);                \
-  template void gemv_dev<T>(long, int, T, const T*, long, const T*, T, T*, cudaStream_t);          \
+  template void mdot<T>(long, int, const T*, long, const T*, T*, T*, cudaStream_t, const T*);      \
+  template void gemv_dev<T>(long, int, T, const T*, long, const T*, T, T*, cudaStream_t, T*);      \
+  template void ritz<T>(long, int, const T*, const T*, const T*, long, const T*, T, T*, T*, T*, T*, T*, cudaStream_t); \
   template void gemv_val<T>(long, int, T, const T*, long, const T*, T, T*, cudaStream_t);          \
   template void rmult<T>(long, int, int, const T*, long, const T*, T*, cudaStream_t);              \
   template void diagsolve<T>(long, const double*, const T*, T*, cudaStream_t);

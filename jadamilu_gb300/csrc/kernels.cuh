@@ -112,17 +112,27 @@ template <class T> void spmv(const SellMatrix<T>& A, const T* x, T* y, cudaStrea
 template <class T> void axpy(long n, T a, const T* x, T* y, cudaStream_t s);
 template <class T> void scal(long n, double a, T* x, cudaStream_t s);
 template <class T> void fill(long n, T v, T* x, cudaStream_t s);
-// out[c] = V(:,c)^H w for c < k (deterministic two-pass reduction); partial
-// needs mdot_partial_size(n,k) entries
+// out[c] = V(:,c)^H w for c < k (deterministic reduction), the last column
+// being xcol when that is given; out may be pinned host memory; partial needs
+// mdot_partial_size(n,k) entries
 long mdot_partial_size(long n, int k);
-template <class T> void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s);
-// w = beta*w + alpha*V*y, y (k <= 64 entries) in device memory or by value
-template <class T> void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, T* w, cudaStream_t s);
-template <class T> void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* y_host, T beta, T* w, cudaStream_t s);
-// The kernels of one fused CG / sQMR iteration (kernels.cu); partial as for mdot.
-// w -= V y (y in device memory, 1 <= k <= 64), *out = x^H w (x null: w^H w)
 template <class T>
-void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s);
+void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s, const T* xcol = nullptr);
+// w = beta*w + alpha*V*y, y (k <= 64 entries) in device memory (copied to the
+// pinned hy when that is given) or by value
+template <class T>
+void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, T* w, cudaStream_t s, T* hy = nullptr);
+template <class T> void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* y_host, T beta, T* w, cudaStream_t s);
+// u = V y, r = W y + a bu (bu = u, or B y), out[0] = r^H r (with B: out[1] = bu^H bu), y on the host
+template <class T>
+void ritz(long n, int k, const T* V, const T* Wv, const T* B, long ld, const T* yh, T a, T* u, T* r, T* bu, T* out,
+          T* partial, cudaStream_t s);
+// The kernels of one fused CG / sQMR iteration (kernels.cu); partial as for mdot.
+// w -= V y (y in device memory, 1 <= k <= 64), *out = x^H w (x null: w^H w), then
+// hsc[0..nsc) = sc[0..nsc) (hsc: pinned host memory)
+template <class T>
+void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s,
+              const T* sc = nullptr, int nsc = 0, T* hsc = nullptr);
 // z += (Re *rho / Re *rho0) p, p = z; rho0 null: p = z unless *rho ends the solve
 template <class T>
 void cg_direction(long n, const T* rho, const T* rho0, bool posdef, T* p, T* z, cudaStream_t s);
