@@ -1022,17 +1022,8 @@ __global__ void __launch_bounds__(RUN_TPB) tail_run_kernel(int m, int s_tail, in
 }
 
 constexpr int TRI_TPB = 256;  // threads per CTA of the tile kernel
+constexpr int kTriDepth = 3;  // units of its chunk that a thread has in flight
 
-// Dense block product y = T x over a set of 64 x 64 tiles (column-major
-// inside a tile), with the reduction inside a thread-block cluster: the CL
-// CTAs of a cluster (8, or 16 where the GPU allows that non-portable size)
-// share one tile row and each streams a contiguous chunk of its tiles
-// (16-byte vectors of V consecutive rows of one tile column per thread;
-// per-column partial sums added in a fixed order) into a 64-vector in its
-// shared memory.  Rank 0 adds the CL vectors in rank order through
-// distributed shared memory and writes the row, so results do not depend on
-// timing.  x must not alias y.  The cluster size is a launch attribute
-// (launch_tri), never left to a default.
 // 16-byte read-only load of data read once per launch (tiles): issued as
 // written, kept in its registers (no re-load at the point of use), no L1 allocation
 __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
@@ -1042,10 +1033,34 @@ __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
                : "l"(p));
   return r;
 }
+
+// Dense block product y = T x over a set of 64 x 64 tiles (column-major
+// inside a tile), with the reduction inside a thread-block cluster: the CL
+// CTAs of a cluster (8, or 16 where the GPU allows that non-portable size)
+// share one tile row and each streams a contiguous chunk of its tiles
+// (16-byte vectors of V consecutive rows of one tile column per thread;
+// per-column partial sums added in a fixed order).  Each CTA puts its
+// 64-vector into rank 0's shared memory; rank 0 adds the CL vectors in rank
+// order and writes the row, so results do not depend on timing.  x must not
+// alias y.  The cluster size is a launch attribute (launch_tri), never left to
+// a default.
+//
+// Bound: the tiles' bytes, for float64 also the FP64 units (2 FMA per SM and
+// cycle), and the chain of tiles of the longest row, ceil(row / CL).  So a
+// thread keeps kTriDepth units of up to four vectors (and their x) in flight,
+// the first ones before it waits for x; the longest rows start first (rev: the
+// longest is the last row); and nothing is requested into L2 ahead.  us per
+// application (GB300), one tile at a time with the rest of the chunk
+// prefetched into L2 -> now: Laplacian 20^3 float64 72.2 -> 69.0, Anderson
+// 28^3 float64 205.7 -> 166.6, float32 70.3 -> 67.5, 40^3 186.6 -> 162.1, 56^3
+// 431 -> 375, 25^3 bfloat16 46.1 -> 47.3.  Two units in flight: 71.8, 172.2,
+// 67.4, 160.3, 377.9, 48.8; three with the prefetch: 69.1, 174.0, 64.6, 178.2,
+// 389.3, 46.3.  Bulk copies through shared memory (four 16 KB stages) were
+// slower for float32 (40^3 201, 56^3 506): the stages cost resident CTAs.
 template <class S, class A, int CL>
 __global__ void __launch_bounds__(TRI_TPB)
-    tri_cluster_kernel(const int4* __restrict__ items, const S* __restrict__ tiles, const A* __restrict__ x, int m,
-                       A* __restrict__ y) {
+    tri_cluster_kernel(const int4* __restrict__ items, bool rev, const S* __restrict__ tiles, const A* __restrict__ x,
+                       int m, A* __restrict__ y) {
   pdl_launch();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -1053,61 +1068,78 @@ __global__ void __launch_bounds__(TRI_TPB)
   constexpr int RG = 64 / V;
   constexpr int CPS = TRI_TPB / RG;
   constexpr int NS = 64 / CPS;
+  constexpr int DEPTH = kTriDepth;
+  constexpr int UN = NS < 4 ? NS : 4;   // vectors per unit
+  constexpr int PER = NS / UN;          // units per tile
   __shared__ A red[CPS][64];
-  __shared__ A mine[64];
-  const int4 it = items[blockIdx.x];
-  const int cnt = it.z;
+  __shared__ A part[CL][64];
+  const int cid = blockIdx.x / CL, ncl = gridDim.x / CL;
+  const int4 it = items[(rev ? ncl - 1 - cid : cid) * CL + blockIdx.x % CL];
+  const int nu = it.z * PER;
   const int rg = threadIdx.x % RG, cs = threadIdx.x / RG;
   A acc[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) acc[v] = A(0);
-  const uint4* tp = reinterpret_cast<const uint4*>(tiles) + (size_t)it.y * (64 * 64 / V);
-  auto load = [&](int k, uint4* buf) {
+  const uint4* tp = reinterpret_cast<const uint4*>(tiles) + (size_t)it.y * (64 * 64 / V) + threadIdx.x;
+  const int c0 = it.w * 64 + cs;
+  auto load = [&](int u, uint4* buf) {
 #pragma unroll
-    for (int sl = 0; sl < NS; ++sl) buf[sl] = ld_stream(tp + (size_t)k * (64 * 64 / V) + (sl * CPS + cs) * RG + rg);
+    for (int sl = 0; sl < UN; ++sl) buf[sl] = ld_stream(tp + ((size_t)u * UN + sl) * TRI_TPB);
   };
-  auto use = [&](int k, const uint4* buf) {
+  auto xload = [&](int u, A* xv) {
 #pragma unroll
-    for (int sl = 0; sl < NS; ++sl) {
-      const int c = (it.w + k) * 64 + sl * CPS + cs;
-      const A xv = c < m ? x[c] : A(0);
-      const S* e = reinterpret_cast<const S*>(&buf[sl]);
-#pragma unroll
-      for (int v = 0; v < V; ++v) acc[v] = fma_(lda<A>(e + v), xv, acc[v]);
+    for (int sl = 0; sl < UN; ++sl) {
+      const int c = c0 + (u * UN + sl) * CPS;
+      xv[sl] = c < m ? x[c] : A(0);
     }
   };
-  // One tile per step.  Measured on GB300 (fp32 factor, Anderson model,
-  // ms per application): 40^3 0.220 -> 0.198 with these loads instead of
-  // __ldg, 50^3 unchanged; issuing the next tile's loads before the current
-  // tile's products made 50^3 slower (0.387 -> 0.410).
-  // the first tile is read, and the others requested into L2, while the
-  // predecessor (which writes x) finishes
-  uint4 b0[NS];
-  if (cnt > 1 && threadIdx.x == 0) l2_prefetch(tp + 64 * 64 / V, sizeof(S) * 64 * 64 * (size_t)(cnt - 1));
-  if (cnt > 0) load(0, b0);
+  uint4 buf[DEPTH][UN];
+  A xv[DEPTH][UN];
+#pragma unroll
+  for (int d = 0; d < DEPTH; ++d)
+    if (d < nu) load(d, buf[d]);
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   pdl_wait();
-  for (int k = 0; k < cnt; ++k) {
-    if (k > 0) load(k, b0);
-    use(k, b0);
+#pragma unroll
+  for (int d = 0; d < DEPTH; ++d)
+    if (d < nu) xload(d, xv[d]);
+  for (int u0 = 0; u0 < nu; u0 += DEPTH) {
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) {
+      const int u = u0 + d;
+      if (u < nu) {
+#pragma unroll
+        for (int sl = 0; sl < UN; ++sl) {
+          const S* e = reinterpret_cast<const S*>(&buf[d][sl]);
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[v] = fma_(lda<A>(e + v), xv[d][sl], acc[v]);
+        }
+        if (u + DEPTH < nu) {
+          load(u + DEPTH, buf[d]);
+          xload(u + DEPTH, xv[d]);
+        }
+      }
+    }
   }
 #pragma unroll
   for (int v = 0; v < V; ++v) red[cs][V * rg + v] = acc[v];
   __syncthreads();
+  A sum = A(0);
   if (threadIdx.x < 64) {
-    A sum = red[0][threadIdx.x];
+    sum = red[0][threadIdx.x];
 #pragma unroll
     for (int j = 1; j < CPS; ++j) sum = sum + red[j][threadIdx.x];
-    mine[threadIdx.x] = sum;
   }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (threadIdx.x < 64) *cl.map_shared_rank(&part[cl.block_rank()][threadIdx.x], 0) = sum;
   cl.sync();
   if (cl.block_rank() == 0 && threadIdx.x < 64) {
-    A sum = A(0);
+    A t = A(0);
 #pragma unroll
-    for (int r = 0; r < CL; ++r) sum = sum + *cl.map_shared_rank(&mine[threadIdx.x], r);
+    for (int r = 0; r < CL; ++r) t = t + part[r][threadIdx.x];
     const int e = it.x * 64 + threadIdx.x;
-    if (e < m) y[e] = sum;
+    if (e < m) y[e] = t;
   }
-  cl.sync();  // the other ranks' shared memory stays alive until rank 0 has read it
 }
 
 // one launch of a cluster kernel: cl CTAs per cluster, PDL as launch_k
@@ -1131,9 +1163,9 @@ static void launch_cl(void (*kern)(Params...), dim3 grid, dim3 block, int cl, cu
 }
 // items are grid-sized multiples of the cluster size (make_cluster_items)
 template <class S, class A>
-static void launch_tri(int items, int cl, const int4* it, const S* tiles, const A* x, int m, A* y, cudaStream_t s) {
-  if (cl == 16) launch_cl(tri_cluster_kernel<S, A, 16>, dim3(items), dim3(TRI_TPB), 16, s, it, tiles, x, m, y);
-  else launch_cl(tri_cluster_kernel<S, A, 8>, dim3(items), dim3(TRI_TPB), 8, s, it, tiles, x, m, y);
+static void launch_tri(int items, int cl, bool lower, const int4* it, const S* tiles, const A* x, int m, A* y, cudaStream_t s) {
+  if (cl == 16) launch_cl(tri_cluster_kernel<S, A, 16>, dim3(items), dim3(TRI_TPB), 16, s, it, lower, tiles, x, m, y);
+  else launch_cl(tri_cluster_kernel<S, A, 8>, dim3(items), dim3(TRI_TPB), 8, s, it, lower, tiles, x, m, y);
 }
 // Whether clusters of 16 tile CTAs can run on the current device: allows the
 // non-portable size on both instantiations' kernel and asks the occupancy
@@ -1338,7 +1370,7 @@ template <class T, class S> void ildl_apply(const DevFactor<S>& F, bool spd, con
       if (B.nt > 0) {
         // right-hand side into xb, then y_B = T xb
         ext(B.m, B.s0, B.ep, B.ei, B.ev, B.nfe, F.xb);
-        launch_tri<S, A>(B.nitf, B.tcl, (const int4*)B.itf, B.tf, (const A*)F.xb, B.m, yb, s);
+        launch_tri<S, A>(B.nitf, B.tcl, true, (const int4*)B.itf, B.tf, (const A*)F.xb, B.m, yb, s);
       } else if (B.nfe > 0) {
         ext(B.m, B.s0, B.ep, B.ei, B.ev, B.nfe, yb);
       }
@@ -1355,7 +1387,7 @@ template <class T, class S> void ildl_apply(const DevFactor<S>& F, bool spd, con
       A* yb = F.y + B.s0;
       if (B.nt > 0) {
         ext(B.m, B.s0, B.bp, B.bi, B.bv, B.nbe, F.xb);
-        launch_tri<S, A>(B.nitb, B.tcl, (const int4*)B.itb, B.tb, (const A*)F.xb, B.m, yb, s);
+        launch_tri<S, A>(B.nitb, B.tcl, false, (const int4*)B.itb, B.tb, (const A*)F.xb, B.m, yb, s);
       } else if (B.nbe > 0) {
         ext(B.m, B.s0, B.bp, B.bi, B.bv, B.nbe, yb);
       }
