@@ -397,45 +397,72 @@ correction:
       // RHO of iteration `it` is kept in device slot kScal + (it & 1), so the
       // next iteration finds its predecessor there.
       T* const scd = W->dsm + kScal;
+      const bool one_launch = device_ops && k::inner_one_ok<T>(N, NEIG + 1, GEP);
       for (;;) {
         ++it;
         if (device_ops) {
-          // The same operations in the same order in six kernels beside the
-          // preconditioner, with RHO, the projection coefficient, the
-          // B-inner product, P^H Q and |R|^2 left on the device and read
-          // back together: one synchronisation per iteration.  The checks on
-          // RHO and P^H Q come after the read; a failed check leaves Q, Z
-          // and R (and P after the first iteration) modified where the plain
-          // sequence stops earlier, and none of them is read after a failed
-          // inner solve.
+          // The same operations in the same order in one kernel beside the
+          // preconditioner (k::inner_one, where the size allows it) or seven,
+          // with RHO, the projection coefficient, the B-inner product, P^H Q
+          // and |R|^2 read back together: one synchronisation per iteration.
+          // The checks on RHO and P^H Q come after the read; a failed check
+          // leaves Q, Z and R (and P after the first iteration) modified
+          // where the plain sequence stops earlier, and none of them is read
+          // after a failed inner solve.
           precond(R, Zv);
           S_.flagcg = true;
           T* rho_d = scd + (it & 1);
           const T* rho0_d = it > 1 ? scd + ((it - 1) & 1) : nullptr;
-          k::mdot<T>(N, NEIG + 1, D(BU), N, D(Zv), W->dsm, W->dpart, S());
-          k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), rho_d, W->dpart, S());
-          k::cg_direction<T>(N, rho_d, rho0_d, POSDEF, D(P), D(Zv), S());
           AXPYALPHA = H(-ETA);
-          matvec_dot(P, Q, Zv, AXPYALPHA, UU, BU, scd + 2);
-          k::gemv_dot<T>(N, 1, D(BU), N, scd + 2, D(Q), D(P), scd + 4, W->dpart, S());
-          k::cg_residual<T>(N, rho_d, scd + 4, D(Q), D(R), scd + 5, scd, 6, W->hsm + kScal, W->dpart, S());
-          sync();
+          H uq, buq;
+          double pq, rr;
           const H* hs = reinterpret_cast<const H*>(W->hsm + kScal);
-          RHO = hre(hs[it & 1]);
+          if (one_launch) {
+            const int parts = inner_one(NEIG + 1, UU, BU, Zv, R, P, AXPYALPHA, it == 1, POSDEF, rho_d, rho0_d);
+            sync();
+            if (hre(hs[4]) != (double)W->one.ticket) {
+              W->reset_barrier();
+              throw std::runtime_error("a grid barrier of the inner iteration ran out");
+            }
+            RHO = hre(hs[0]);
+            uq = hs[1];
+            buq = hs[2];
+            pq = hre(hs[3]);
+            rr = k::md_sum_host(W->hpart, parts);
+          } else {
+            k::mdot<T>(N, NEIG + 1, D(BU), N, D(Zv), W->dsm, W->dpart, S());
+            double* const be = reinterpret_cast<double*>(scd + 6);  // this iteration's two update scalars
+            double* const al = reinterpret_cast<double*>(scd + 7);
+            k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), rho_d, W->dpart, S(), nullptr, 0, nullptr, nullptr,
+                           rho0_d, rho0_d ? be : nullptr);
+            k::cg_direction<T>(N, rho_d, rho0_d ? be : nullptr, POSDEF, D(P), D(Zv), S());
+            matvec_shift(P, Q, Zv, AXPYALPHA);
+            k::mdot<T>(N, 1, D(UU), N, D(Q), scd + 2, W->dpart, S());
+            if (GEP) k::mdot<T>(N, 1, D(BU), N, D(Q), scd + 3, W->dpart, S());
+            k::gemv_dot<T>(N, 1, D(BU), N, scd + 2, D(Q), D(P), scd + 4, W->dpart, S(), nullptr, 0, nullptr, rho_d,
+                           nullptr, al);
+            k::cg_residual<T>(N, al, D(Q), D(R), scd + 5, scd, 6, W->hsm + kScal, W->dpart, S());
+            sync();
+            RHO = hre(hs[it & 1]);
+            uq = hs[2];
+            buq = hs[3];
+            pq = hre(hs[4]);
+            rr = hre(hs[5]);
+          }
           if (POSDEF && RHO <= 0) {
             std::fprintf(stderr, " Non fatal bug: the preconditioner is not positive definite\n");
             fail = true;
             break;
           }
           if (RHO == 0) { fail = true; break; }
-          if (GEP) AXPYALPHA = hs[3] / (NBU * NBU);
-          X[NP] = hs[2];
+          if (GEP) AXPYALPHA = buq / (NBU * NBU);
+          X[NP] = uq;
           ALPRHO = hre(X[NP]);
           ITER++;
-          alpha_cg = hre(hs[4]);
+          alpha_cg = pq;
           if ((POSDEF && alpha_cg <= 0) || alpha_cg == 0) { fail = true; break; }
           alpha_cg = RHO / alpha_cg;
-          GK = std::sqrt(rl(W->hsm[kScal + 5]));
+          GK = std::sqrt(rr);
         } else {
         precond(R, Zv);
         S_.flagcg = true;

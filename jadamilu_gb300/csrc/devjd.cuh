@@ -44,6 +44,15 @@ template <class T> struct Workspace {
   T* hsm = nullptr;    // pinned host mirror
   T* dpart = nullptr;  // reduction partials
   T* dtmp = nullptr;   // N x 32 scratch for restarts
+  // the one-launch inner iteration: partial sums it leaves for the host, its
+  // grid barrier's counter and what the host knows it holds
+  double* hpart = nullptr;
+  unsigned* dbar = nullptr;
+  k::OneState one;
+  void reset_barrier() {
+    CK(cudaMemsetAsync(dbar, 0, sizeof(unsigned), st));
+    one.base = 0;
+  }
   bool own_stream = false;
   void set_stream(cudaStream_t s) {
     if (own_stream && st) cudaStreamDestroy(st);
@@ -58,6 +67,9 @@ template <class T> struct Workspace {
     if (!dsm) {
       CK(cudaMalloc(&dsm, sizeof(T) * 512));
       CK(cudaMallocHost(&hsm, sizeof(T) * 512));
+      CK(cudaMallocHost(&hpart, sizeof(double) * k::kMaxPartials));
+      CK(cudaMalloc(&dbar, sizeof(unsigned)));
+      reset_barrier();
     }
     if (lx > cap_x) {
       if (dX) CK(cudaFree(dX));
@@ -85,10 +97,14 @@ template <class T> struct Workspace {
     if (dX) cudaFree(dX);
     if (dsm) cudaFree(dsm);
     if (hsm) cudaFreeHost(hsm);
+    if (hpart) cudaFreeHost(hpart);
+    if (dbar) cudaFree(dbar);
     if (dpart) cudaFree(dpart);
     if (dtmp) cudaFree(dtmp);
     if (own_stream && st) cudaStreamDestroy(st);
     dX = dsm = hsm = dpart = dtmp = nullptr;
+    hpart = nullptr;
+    dbar = nullptr;
     st = nullptr;
     own_stream = false;
     cap_x = cap_tmp = cap_part = 0;
@@ -119,9 +135,11 @@ template <class T> struct DevJd {
   // which: 1 = A x (and B x for GEP), 3 = A x, 4 = B x; offsets into X
   std::function<void(int, long, long, long)> matvec;
   std::function<void(long, long)> precond;  // (rhs, sol)
-  // built-in matrix: y = A x + a x (GEP: yb = B x, y = A x + a yb), out[0] = d0^H y
-  // and for GEP out[1] = d1^H y, in one kernel (offsets x, y, yb, d0, d1)
-  std::function<void(long, long, long, H, long, long, T*)> matvec_dot;
+  // built-in matrix: y = A x + a x (GEP: yb = B x, y = A x + a yb) in one kernel (offsets x, y, yb)
+  std::function<void(long, long, long, H)> matvec_shift;
+  // built-in matrix: the whole inner iteration outside the preconditioner in
+  // one launch (k columns from U and BU; offsets z, r, p), see k::inner_one
+  std::function<int(int, long, long, long, long, long, H, bool, bool, T*, const T*)> inner_one;
   std::function<void(int, int, int, double, double)> on_step;  // progress printer (may be empty)
   StopStateD<T> st;
   Lcg48d rng;

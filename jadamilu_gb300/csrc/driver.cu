@@ -603,6 +603,17 @@ void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, A
 template <class T> struct LowOf { using type = float; using bf = __nv_bfloat16; };
 template <> struct LowOf<zc> { using type = cc; using bf = bc; };
 
+// Throws when a kernel before it on st gave up a bounded wait (its results are
+// then not to be used).  host: pinned memory for the flag.
+static void check_waits(cudaStream_t st, int* host) {
+  int* flag = k::wait_expired_flag();
+  CK(cudaMemcpyAsync(host, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (*host == 0) return;
+  CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  throw std::runtime_error("a bounded wait inside a kernel ran out");
+}
+
 // ------------------------------------------------------- global state ----
 
 template <class T> struct Global {
@@ -935,10 +946,16 @@ template <class T> struct PjdRun {
     if (which == 1 || which == 3) k::spmv<T>(g.A, jd.D(x), jd.D(y), g.W.st);
     if ((which == 1 || which == 4) && gep) k::spmv<T>(g.Bm, jd.D(x), jd.D(by), g.W.st);
   }
-  void builtin_mv_dot(long x, long y, long yb, typename HostOf<T>::type a, long d0, long d1, T* out) {
+  void builtin_mv_shift(long x, long y, long yb, typename HostOf<T>::type a) {
     g.n_matvec++;
-    k::spmv_dot<T>(g.A, gep ? &g.Bm : nullptr, todev(a), jd.D(x), jd.D(y), jd.D(yb), jd.D(d0), jd.D(d1), out, g.W.dpart,
-                   g.W.st);
+    k::spmv_shift<T>(g.A, gep ? &g.Bm : nullptr, todev(a), jd.D(x), jd.D(y), jd.D(yb), g.W.st);
+  }
+  int builtin_inner(int cols, long U, long BU, long z, long r, long p, typename HostOf<T>::type eta, bool first,
+                    bool posdef, T* rho, const T* rho0) {
+    g.n_matvec++;
+    return k::inner_one<T>(g.A, gep ? &g.Bm : nullptr, cols, jd.D(U), jd.D(BU), jd.D(z), jd.D(r), jd.D(p),
+                           todev(eta), first, posdef, rho, rho0, g.W.hsm + DevJd<T>::kScal,
+                           g.W.dpart + k::kPartialHead, g.W.hpart, g.W.dbar, g.W.one, g.W.st);
   }
   void precond(long rhs, long sol);
 };
@@ -1162,8 +1179,11 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
   jd.precond = [&R](long r, long s) { R.precond(r, s); };
   jd.device_ops = !user_mv && g_opt.fuse_inner != 0;
   if (jd.device_ops)
-    jd.matvec_dot = [&R](long x, long y, long yb, typename HostOf<T>::type a, long d0, long d1, T* out) {
-      R.builtin_mv_dot(x, y, yb, a, d0, d1, out);
+    jd.matvec_shift = [&R](long x, long y, long yb, typename HostOf<T>::type a) { R.builtin_mv_shift(x, y, yb, a); };
+  if (jd.device_ops)
+    jd.inner_one = [&R](int k, long U, long BU, long z, long r, long p, typename HostOf<T>::type eta,
+                        bool first, bool posdef, T* rho, const T* rho0) {
+      return R.builtin_inner(k, U, BU, z, r, p, eta, first, posdef, rho, rho0);
     };
   if (R.P.pr >= 2)
     jd.on_step = [](int conv, int step, int k, double th, double v) {
@@ -1186,7 +1206,7 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
     long BX = (long)R.NW * n + (long)std::min(MADSPACE, n) * n * 2;
     CK(cudaMemcpyAsync(X + BX, g.W.dX + BX, sizeof(T) * (size_t)n * nv, cudaMemcpyDeviceToHost, g.W.st));
   }
-  CK(cudaStreamSynchronize(g.W.st));
+  check_waits(g.W.st, reinterpret_cast<int*>(g.W.hsm));
   const double t2 = wall();
   print_table<T>(R.P, EIGS, RES, *NEIG, *ITER, *GAP, *INFO, t2 - t1);
   if (R.P.pr >= 1)

@@ -107,6 +107,8 @@ long long launch_count();
 // programmatic dependent launch between the preconditioner's kernels (default on)
 void set_pdl(bool on);
 void add_launches(long long n);
+// device flag that a kernel sets when a bounded wait inside it ran out
+int* wait_expired_flag();
 
 template <class T> void spmv(const SellMatrix<T>& A, const T* x, T* y, cudaStream_t s);
 template <class T> void axpy(long n, T a, const T* x, T* y, cudaStream_t s);
@@ -115,6 +117,7 @@ template <class T> void fill(long n, T v, T* x, cudaStream_t s);
 // out[c] = V(:,c)^H w for c < k (deterministic reduction), the last column
 // being xcol when that is given; out may be pinned host memory; partial needs
 // mdot_partial_size(n,k) entries
+constexpr int kPartialHead = 8;  // entries before the partials: the arrival counters
 long mdot_partial_size(long n, int k);
 template <class T>
 void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s, const T* xcol = nullptr);
@@ -129,21 +132,38 @@ void ritz(long n, int k, const T* V, const T* Wv, const T* B, long ld, const T* 
           T* partial, cudaStream_t s);
 // The kernels of one fused CG / sQMR iteration (kernels.cu); partial as for mdot.
 // w -= V y (y in device memory, 1 <= k <= 64), *out = x^H w (x null: w^H w), then
-// hsc[0..nsc) = sc[0..nsc) (hsc: pinned host memory)
+// hsc[0..nsc) = sc[0..nsc) (hsc: pinned host memory) and *ratio = Re *out / Re *rden, or Re *rnum / Re *out
 template <class T>
 void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s,
-              const T* sc = nullptr, int nsc = 0, T* hsc = nullptr);
-// z += (Re *rho / Re *rho0) p, p = z; rho0 null: p = z unless *rho ends the solve
+              const T* sc = nullptr, int nsc = 0, T* hsc = nullptr, const T* rnum = nullptr, const T* rden = nullptr,
+              double* ratio = nullptr);
+// z += *be p, p = z; be null: p = z unless *rho ends the solve
 template <class T>
-void cg_direction(long n, const T* rho, const T* rho0, bool posdef, T* p, T* z, cudaStream_t s);
-// y = A x + a x, out[0] = d0^H y; with B: yb = B x, y = A x + a yb, out[0..1] = d0^H y, d1^H y
+void cg_direction(long n, const T* rho, const double* be, bool posdef, T* p, T* z, cudaStream_t s);
+// y = A x + a x; with B: yb = B x, y = A x + a yb
 template <class T>
-void spmv_dot(const SellMatrix<T>& A, const SellMatrix<T>* B, T a, const T* x, T* y, T* yb, const T* d0, const T* d1,
-              T* out, T* partial, cudaStream_t s);
-// r -= (Re *num / Re *den) q, *out = r^H r, then hsc[0..nsc) = sc[0..nsc) (hsc: pinned host memory)
+void spmv_shift(const SellMatrix<T>& A, const SellMatrix<T>* B, T a, const T* x, T* y, T* yb, cudaStream_t s);
+// r -= *al q, *out = r^H r, then hsc[0..nsc) = sc[0..nsc) (hsc: pinned host memory)
 template <class T>
-void cg_residual(long n, const T* num, const T* den, const T* q, T* r, T* out, const T* sc, int nsc, T* hsc, T* partial,
+void cg_residual(long n, const double* al, const T* q, T* r, T* out, const T* sc, int nsc, T* hsc, T* partial,
                  cudaStream_t s);
+// The kernels from mdot(BU, z) to cg_residual as one launch (one per stream at a time), where the rows and columns
+// allow it: r and p as there, z = B p with B (else left alone), rho (device, this iteration's), and on the host after
+// the stream has synchronised hsc[0..4] = rho, U^H q, BU^H q (with B), p^H q, st.ticket (as the call left it; anything
+// else: a barrier gave up) and hpart[0..g) the partials of r^H r, g the return value, to be added by md_sum_host.
+// part: inner_one_partials(n, k) entries; bar: a counter that starts at zero, with st.base = 0, and is only used here.
+struct OneState {
+  unsigned base = 0;    // what the barrier counter holds
+  unsigned ticket = 0;  // launches so far
+};
+template <class T> bool inner_one_ok(long n, int k, bool gep);
+int inner_one_partials(long n, int k);
+constexpr int kMaxPartials = 152 * 8;  // most CTAs of a reduction
+double md_sum_host(const double* p, int g);
+template <class T>
+int inner_one(const SellMatrix<T>& A, const SellMatrix<T>* B, int k, const T* U, const T* BU, T* z, T* r, T* p, T eta,
+              bool first, bool posdef, T* rho, const T* rho0, T* hsc, T* part, double* hpart, unsigned* bar, OneState& st,
+              cudaStream_t s);
 // smooth: x2 = sc (x2 + a p), x += x2 (first: x2 = sc p, x = x2); else x += a p (first: from zero); bt, when given,
 // += al bp (first: from zero)
 template <class T>
