@@ -116,7 +116,7 @@ template <> struct StoreOf<bc> {
 
 template <class S> void free_factor(DevFactor<S>& F) {
   void* ps[] = {F.orig, F.lp,  F.li,  F.lx,  F.up,  F.ui,  F.ux,    F.brows, F.blk,   F.partner, F.dv,
-                F.dof,  F.av,  F.aof, F.y,   F.dfptr, F.dbptr, F.rhs_in, F.sol_out, F.tep, F.tei, F.tev,
+                F.dof,  F.av,  F.aof, F.y,   F.dfptr, F.dbptr, F.tep, F.tei, F.tev,
                 F.tip,  F.tii, F.tiv, F.dtfptr, F.tbp, F.tbi, F.tbv, F.dtbptr, F.tbrows,
                 F.part, F.xb, F.perm, F.fpp, F.fpi, F.fpx, F.fhp, F.fhi, F.fhx, F.cy, F.cyb, F.ct};
   for (void* p : ps)
@@ -129,6 +129,8 @@ template <class S> void free_factor(DevFactor<S>& F) {
   }
   for (auto& g : F.graph)
     if (g) cudaGraphExecDestroy(g);
+  for (auto& g : F.graph_def)
+    if (g) cudaGraphDestroy(g);
   F = DevFactor<S>();
 }
 
@@ -201,14 +203,13 @@ struct DeviceMalloc {
 };
 
 template <class S, class H, class Alloc>
-void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Alloc alloc, bool graph_io);
+void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Alloc alloc);
 
 template <class S, class H, class Alloc = DeviceMalloc>
-void upload_factor(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Alloc alloc = Alloc(),
-                   bool graph_io = true) {
+void upload_factor(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Alloc alloc = Alloc()) {
   free_factor(D);
   if (F.coupling == 1) {
-    upload_coupled(F, D, st, alloc, graph_io);
+    upload_coupled(F, D, st, alloc);
     return;
   }
   const int n = F.n;
@@ -485,10 +486,6 @@ void upload_factor(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Al
   }
   if (max_items > 0) D.xb = (A*)alloc(sizeof(A) * max_items);
   D.y = (A*)alloc(sizeof(A) * std::max(1, n));
-  if (graph_io) {  // the input and output vectors of the captured application graph
-    D.rhs_in = alloc(sizeof(zc) * std::max(1, n));
-    D.sol_out = alloc(sizeof(zc) * std::max(1, n));
-  }
   k::ildl_plan(D, lp, up, brs);
   k::ildl_plan_bwd0(D, up, brs);
   CK(cudaStreamSynchronize(st));
@@ -508,7 +505,7 @@ void upload_factor(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Al
 // F^H are stored as CSR over elimination steps, plus the work vectors of the
 // composed application (k::ildl_apply).
 template <class S, class H, class Alloc>
-void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Alloc alloc, bool graph_io) {
+void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, Alloc alloc) {
   const int n = F.n;
   const int nl = (int)F.level_start.size() - 1;
   D.n = n;
@@ -537,7 +534,7 @@ void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, A
     sub.ainv.assign(F.ainv.begin() + a, F.ainv.begin() + e);
     sub.aoff.assign(F.aoff.begin() + a, F.aoff.begin() + e);
     sub.level_start = {0, m};
-    upload_factor(sub, D.lev[l], st, alloc, false);
+    upload_factor(sub, D.lev[l], st, alloc);
     // each level below the last is solved twice per application
     const int mult = l + 1 < nl ? 2 : 1;
     D.nnz_l += D.lev[l].nnz_l;
@@ -593,10 +590,6 @@ void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, A
   D.cy = alloc(sizeof(H) * std::max(1, n));
   D.cyb = alloc(sizeof(H) * std::max(1, n));
   D.ct = alloc(sizeof(H) * std::max(1, n));
-  if (graph_io) {
-    D.rhs_in = alloc(sizeof(zc) * std::max(1, n));
-    D.sol_out = alloc(sizeof(zc) * std::max(1, n));
-  }
   CK(cudaStreamSynchronize(st));  // the host arrays are released next
 }
 
@@ -2119,10 +2112,9 @@ JDG_API int jdgpu_dildl_apply_noalloc(int n, const int* ia, const int* ja, const
     DevFactor<double> Fd;
     DevFactor<float> Fs;
     DevFactor<__nv_bfloat16> Fb;
-    // applied without the captured graph: no graph input/output vectors
-    if (precision == 1) upload_factor(F, Fs, st, bump, false);
-    else if (precision == 2) upload_factor(F, Fb, st, bump, false);
-    else upload_factor(F, Fd, st, bump, false);
+    if (precision == 1) upload_factor(F, Fs, st, bump);
+    else if (precision == 2) upload_factor(F, Fb, st, bump);
+    else upload_factor(F, Fd, st, bump);
     for (int r = 0; r < nrhs; ++r) {
       CK(cudaMemcpy(db, b + (size_t)r * n, sizeof(double) * n, cudaMemcpyHostToDevice));
       if (precision == 1) k::ildl_apply<double, float>(Fs, spd != 0, db, dx, st);

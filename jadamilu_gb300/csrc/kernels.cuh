@@ -56,8 +56,6 @@ template <class S> struct DevFactor {
   signed char* blk = nullptr; int* partner = nullptr;
   S *dv = nullptr, *dof = nullptr, *av = nullptr, *aof = nullptr;  // D^{-1} and |D|^{-1}
   A* y = nullptr;                            // work vector
-  // captured launch sequence of one application (per spd flag), reading
-  // rhs_in and writing sol_out
   // Tail: rows s >= s_tail (the deepest forward levels, m_tail rows) are
   // solved by one CTA with the tail of y in shared memory.  Forward: the
   // entries of tail rows that point below s_tail ("external") are applied by
@@ -77,10 +75,15 @@ template <class S> struct DevFactor {
   A* xb = nullptr;                           // right-hand side of the dense block being solved
   int64_t sweep_entries = 0;                 // L / L^H entries the two level sweeps read
   double tile_bytes = 0;                     // bytes of both tile sets
+  // captured launch sequence of one application (per spd flag)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   long long graph_kernels[2] = {0, 0};
-  void* rhs_in = nullptr;
-  void* sol_out = nullptr;
+  // the graph it was made from, its first and last node, and the vectors they
+  // read and write in the executable graph
+  cudaGraph_t graph_def[2] = {nullptr, nullptr};
+  cudaGraphNode_t graph_in[2] = {nullptr, nullptr}, graph_out[2] = {nullptr, nullptr};
+  const void* graph_b[2] = {nullptr, nullptr};
+  void* graph_x[2] = {nullptr, nullptr};
   // Multilevel form with coupling blocks (IldlcFactor::coupling == 1): one
   // sub-factor per level (rows in elimination order, identity permutation),
   // the blocks F (rows: steps of the level's pivots; columns: later steps;
@@ -175,8 +178,7 @@ template <class T> void rmult(long n, int K, int keep, const T* V, long ldv, con
 template <class T> void diagsolve(long n, const double* d, const T* rhs, T* sol, cudaStream_t s);
 // preconditioner application  x = P (L D L^H)^{-1} P^T b  (|D| when spd)
 template <class T, class S> void ildl_apply(const DevFactor<S>& F, bool spd, const T* b, T* x, cudaStream_t s);
-// the same through the captured graph (builds it on first use); F.rhs_in and
-// F.sol_out must hold n entries of T
+// the same through the captured graph (builds it on first use)
 template <class T, class S> void ildl_apply_graph(DevFactor<S>& F, bool spd, const T* b, T* x, cudaStream_t s);
 // lanes of a warp that share one row of a given mean length in the row kernels
 int lanes_per_row(double entries_per_row);
