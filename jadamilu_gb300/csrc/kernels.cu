@@ -1142,14 +1142,33 @@ __device__ __forceinline__ void ent_load(EntBatch<A, U>& b, int64_t q, int64_t e
     }
   }
 }
-template <class A, int U> __device__ __forceinline__ A ent_use(const EntBatch<A, U>& b, const A* y, A acc) {
+// nu: how many entries of the batch any lane of the warp may have (a bound that
+// is the same in all lanes lets the warp skip the rest).
+template <class A, int U>
+__device__ __forceinline__ A ent_use(const EntBatch<A, U>& b, const A* y, A acc, int nu = U) {
   A w[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) w[u] = b.c[u] >= 0 ? y[b.c[u]] : A(0);
+  for (int u = 0; u < U; ++u) w[u] = u < nu && b.c[u] >= 0 ? y[b.c[u]] : A(0);
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    if (b.c[u] >= 0) acc = fma_(b.v[u], w[u], acc);
+    if (u < nu && b.c[u] >= 0) acc = fma_(b.v[u], w[u], acc);
   return acc;
+}
+// The longest of a warp's rows, and the tree over the LANES lanes of a row
+// whose sums lie in its first lanes: steps that would only add zeros (rows of
+// at most o entries leave the lanes from o on empty) are left out.  Short rows
+// are the rule in the first and last levels, and a float64 addition occupies
+// the SM's FP64 unit for 16 cycles per warp whether its lanes are zero or not.
+// us per application (GB300): tridiagonal n = 1000 28.7 -> 22.6, FEM 384^2 291
+// -> 276, Anderson 56^3 350 -> 339, 40^3 151 -> 149, Laplacian 20^3 58.2 -> 56.7.
+__device__ __forceinline__ int warp_longest(int64_t len) {
+  return __reduce_max_sync(0xffffffffu, (int)(len < 0 ? 0 : len < 4096 ? len : 4096));
+}
+template <int LANES, class A> __device__ __forceinline__ A row_sum(A v, int longest) {
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1)
+    if (o < longest) v = v + shfl_xor_any(v, o);
+  return v;
 }
 // entries [q, e) of a row beyond its first batch, into L2 ahead of use
 template <class S>
@@ -1185,9 +1204,10 @@ __device__ __forceinline__ A ent_dot(int64_t q, int64_t e, int step, const int* 
 // 163.5, FEM 384^2 302 -> 299; batches of eight instead: 362, 70.7, 184, 339.
 template <bool NC, int U, class A, class S>
 __device__ __forceinline__ A ent_pipe(EntBatch<A, U>& b, int64_t q, int64_t e, int step, const int* __restrict__ ci,
-                                      const S* __restrict__ cv, EntBatch<A, U>& nx, const A* y) {
+                                      const S* __restrict__ cv, EntBatch<A, U>& nx, const A* y, int nu) {
   A acc = A(0);
   q += (int64_t)U * step;  // nx holds the batch at q when q < e
+  if (nu < U) return ent_use(b, y, acc, nu);
   while (q < e) {
     acc = ent_use(b, y, acc);
     b = nx;
@@ -1252,6 +1272,8 @@ constexpr int RUN_TPB = 1024;
 constexpr int RUN_WARPS = RUN_TPB / 32;
 // A level with R < 32 rows gives each row 32/R warps; their partial sums are
 // added in a fixed order after a barrier, so results do not depend on timing.
+// Bound for float64: the one SM's FP64 unit, which is why sums over empty lanes
+// and warps are left out (row_sum).
 template <class S, class A>
 __global__ void __launch_bounds__(RUN_TPB) ildl_run_kernel(int l0, int l1, const int* __restrict__ lptr,
                                                           const int* __restrict__ rows, const int64_t* __restrict__ rp,
@@ -1262,32 +1284,47 @@ __global__ void __launch_bounds__(RUN_TPB) ildl_run_kernel(int l0, int l1, const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int l = l0; l < l1; ++l) {
     const int lo = lptr[l], hi = lptr[l + 1], R = hi - lo;
+    // the sum of this warp's entries of row s: from entry `off` of the row on, every `step`
+    auto sum = [&](int s, int off, int step) {
+      const int64_t b = rp[s], e = rp[s + 1];
+      const int len = warp_longest(e - b - off), nu = (len + step - 1) / step;
+      A acc;
+      if (nu <= kUnr) {
+        EntBatch<A, kUnr> first;
+        ent_load<false>(first, b + off + lane, e, step, ci, cv);
+        acc = ent_use(first, (const A*)y, A(0), nu);
+      } else {
+        acc = ent_dot<false>(b + off + lane, e, step, ci, cv, (const A*)y, A(0));
+      }
+      return row_sum<32>(acc, len);
+    };
     if (R >= RUN_WARPS) {
       for (int t = lo + warp; t < hi; t += RUN_WARPS) {
         const int s = rows ? rows[t] : t;
-        const int64_t b = rp[s], e = rp[s + 1];
-        A acc = ent_dot<false>(b + lane, e, 32, ci, cv, (const A*)y, A(0));
-        acc = wsum(acc);
-        if (lane == 0) y[s] = y[s] - acc;
+        const A own = y[s];
+        const A acc = sum(s, 0, 32);
+        if (lane == 0) y[s] = own - acc;
       }
       __syncthreads();
     } else {
       int G = RUN_WARPS / R;
       G = 1 << (31 - __clz(G));
       const int slot = warp / G, sub = warp % G;
-      A acc = A(0);
-      int s = -1;
+      int s = -1, parts = 0;  // the row and how many of its G warps have entries
+      A own = A(0);
       if (slot < R) {
         s = rows ? rows[lo + slot] : lo + slot;
-        acc = ent_dot<false>(rp[s] + sub * 32 + lane, rp[s + 1], 32 * G, ci, cv, (const A*)y, acc);
+        own = y[s];
+        parts = (warp_longest(rp[s + 1] - rp[s]) + 31) / 32;
+        parts = parts < G ? parts : G;
+        const A acc = sub < parts ? sum(s, sub * 32, 32 * G) : A(0);
+        if (lane == 0) part[warp] = acc;
       }
-      acc = wsum(acc);
-      if (lane == 0) part[warp] = acc;
       __syncthreads();
       if (slot < R && sub == 0 && lane == 0) {
         A t = part[warp];
-        for (int j = 1; j < G; ++j) t = t + part[warp + j];
-        y[s] = y[s] - t;
+        for (int j = 1; j < parts; ++j) t = t + part[warp + j];
+        y[s] = own - t;
       }
       __syncthreads();
     }
@@ -1318,12 +1355,13 @@ __global__ void __launch_bounds__(WIDE_TPB) ildl_wide_kernel(int lo, int hi, con
     if (lane == 0) prefetch_rest(b + kUnr * LANES, e, ci, cv);
   }
   EntBatch<A, kUnr> first, second;
+  const int longest = warp_longest(ok ? e - b + lane : 0);
   ent_load<false>(first, b, e, LANES, ci, cv);
   ent_load<false>(second, b + kUnr * LANES, e, LANES, ci, cv);
   pdl_wait();
   const A own = ok && lane == 0 ? y[s] : A(0);  // requested with the gathers, not after the sum
-  A acc = ent_pipe<false, kUnr>(first, b, e, LANES, ci, cv, second, (const A*)y);
-  for (int o = LANES / 2; o > 0; o >>= 1) acc = acc + shfl_xor_any(acc, o);
+  A acc = ent_pipe<false, kUnr>(first, b, e, LANES, ci, cv, second, (const A*)y, (longest + LANES - 1) / LANES);
+  acc = row_sum<LANES>(acc, longest);
   if (ok && lane == 0) y[s] = own - acc;
 }
 
@@ -1349,12 +1387,13 @@ __global__ void __launch_bounds__(WIDE_TPB) tail_ext_kernel(int m, int s_tail, c
     if (lane == 0) prefetch_rest(b + U * LANES, e, ci, cv);
   }
   EntBatch<A, U> first, second;
+  const int longest = warp_longest(t < m ? e - b + lane : 0);
   ent_load<NC>(first, b, e, LANES, ci, cv);
   ent_load<NC>(second, b + U * LANES, e, LANES, ci, cv);
   pdl_wait();
   const A own = t < m && lane == 0 ? y[s_tail + t] : A(0);
-  A acc = ent_pipe<NC, U>(first, b, e, LANES, ci, cv, second, y);
-  for (int o = LANES / 2; o > 0; o >>= 1) acc = acc + shfl_xor_any(acc, o);
+  A acc = ent_pipe<NC, U>(first, b, e, LANES, ci, cv, second, y, (longest + LANES - 1) / LANES);
+  acc = row_sum<LANES>(acc, longest);
   if (t < m && lane == 0) out[t] = own - acc;
 }
 template <class S, class A>
