@@ -240,9 +240,9 @@ main_loop:
     // GEP's harmonic extraction it needs |B u| first
     ritz_late = !(GEP && ISERCH == 2);
     if (!ritz_late) {
-      gemvn(N, (int)J, H(1), VV, N, X + YY, H(0), UU);
-      gemvn(N, (int)J, H(1), WW, N, X + YY, H(0), REIG);
-      gemvn(N, (int)J, H(1), BV, N, X + YY, H(0), BU);
+      gemvn(N, (int)J, 1.0, VV, N, X + YY, 0.0, UU);
+      gemvn(N, (int)J, 1.0, WW, N, X + YY, 0.0, REIG);
+      gemvn(N, (int)J, 1.0, BV, N, X + YY, 0.0, BU);
     }
   } else {
     ritz_late = false;
@@ -270,7 +270,7 @@ main_loop:
   if (ritz_late) {
     T y[32];
     for (long c = 0; c < J; ++c) y[c] = todev(X[YY + c]);
-    k::ritz<T>(N, (int)J, D(VV), D(WW), GEP ? D(BV) : nullptr, N, y, todev(H(-THMT)), D(UU), D(REIG),
+    k::ritz<T>(N, (int)J, D(VV), D(WW), GEP ? D(BV) : nullptr, N, y, -THMT, D(UU), D(REIG),
                GEP ? D(BU) : nullptr, W->hsm, W->dpart, S());
     sync();
     NREIG = std::sqrt(rl(W->hsm[0]));
@@ -418,7 +418,7 @@ correction:
           double pq, rr;
           const H* hs = reinterpret_cast<const H*>(W->hsm + kScal);
           if (one_launch) {
-            const int parts = inner_one(NEIG + 1, UU, BU, Zv, R, P, AXPYALPHA, it == 1, POSDEF, rho_d, rho0_d);
+            const int parts = inner_one(NEIG + 1, UU, BU, Zv, R, P, -ETA, it == 1, POSDEF, rho_d, rho0_d);
             sync();
             if (hre(hs[4]) != (double)W->one.ticket) {
               W->reset_barrier();
@@ -436,7 +436,7 @@ correction:
             k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), rho_d, W->dpart, S(), nullptr, 0, nullptr, nullptr,
                            rho0_d, rho0_d ? be : nullptr);
             k::cg_direction<T>(N, rho_d, rho0_d ? be : nullptr, POSDEF, D(P), D(Zv), S());
-            matvec_shift(P, Q, Zv, AXPYALPHA);
+            matvec_shift(P, Q, Zv, -ETA);
             k::mdot<T>(N, 1, D(UU), N, D(Q), scd + 2, W->dpart, S());
             if (GEP) k::mdot<T>(N, 1, D(BU), N, D(Q), scd + 3, W->dpart, S());
             k::gemv_dot<T>(N, 1, D(BU), N, scd + 2, D(Q), D(P), scd + 4, W->dpart, S(), nullptr, 0, nullptr, rho_d,
@@ -507,8 +507,8 @@ correction:
           GGK2 = GGK2 * TTK2 * (1 / (1 + TTK2));
         }
         const double CK2 = 1 / (1 + TTK2);
-        k::cg_iterate<T>(N, !POSDEF, it == 1, todev(H(POSDEF ? alpha_cg : alpha_cg / TTK2M)),
-                         it == 1 ? alpha_cg * CK2 : TTK2M * CK2, D(P), D(X2), D(Xc), todev(H(alpha_cg)), D(Zv),
+        k::cg_iterate<T>(N, !POSDEF, it == 1, POSDEF ? alpha_cg : alpha_cg / TTK2M,
+                         it == 1 ? alpha_cg * CK2 : TTK2M * CK2, D(P), D(X2), D(Xc), alpha_cg, D(Zv),
                          GEP ? D(BTv) : nullptr, S());
         if (FTFLG) IFO = (ISERCH == 2) ? -2 : -1;
         if (FTFLG && GEP) AXPYBETA = reinterpret_cast<const H*>(W->hsm)[kLate] / (NBU * NBU);

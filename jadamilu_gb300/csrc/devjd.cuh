@@ -136,10 +136,10 @@ template <class T> struct DevJd {
   std::function<void(int, long, long, long)> matvec;
   std::function<void(long, long)> precond;  // (rhs, sol)
   // built-in matrix: y = A x + a x (GEP: yb = B x, y = A x + a yb) in one kernel (offsets x, y, yb)
-  std::function<void(long, long, long, H)> matvec_shift;
+  std::function<void(long, long, long, double)> matvec_shift;
   // built-in matrix: the whole inner iteration outside the preconditioner in
   // one launch (k columns from U and BU; offsets z, r, p), see k::inner_one
-  std::function<int(int, long, long, long, long, long, H, bool, bool, T*, const T*)> inner_one;
+  std::function<int(int, long, long, long, long, long, double, bool, bool, T*, const T*)> inner_one;
   std::function<void(int, int, int, double, double)> on_step;  // progress printer (may be empty)
   StopStateD<T> st;
   Lcg48d rng;
@@ -198,13 +198,13 @@ template <class T> struct DevJd {
     }
   }
   // X(w) = beta X(w) + alpha X(V) y, y on the host
-  void gemvn(long n, int kc, H alpha, long V, long ldv, const H* y, H beta, long w) {
+  void gemvn(long n, int kc, double alpha, long V, long ldv, const H* y, double beta, long w) {
     std::vector<T> yd(std::max(kc, 1));
     for (int c = 0; c < kc; ++c) yd[c] = todev(y[c]);
     for (int c0 = 0; c0 < std::max(kc, 1); c0 += 64) {
       int kk = std::min(64, kc - c0);
-      H b = (c0 == 0) ? beta : H(1);
-      k::gemv_val<T>(n, std::max(kk, 0), todev(alpha), D(V + (long)c0 * ldv), ldv, yd.data() + c0, todev(b), D(w), S());
+      const double b = (c0 == 0) ? beta : 1.0;
+      k::gemv_val<T>(n, std::max(kk, 0), alpha, D(V + (long)c0 * ldv), ldv, yd.data() + c0, b, D(w), S());
       if (kc <= 0) break;
     }
   }
@@ -224,7 +224,7 @@ template <class T> struct DevJd {
       // given, is filled after the next synchronisation by repgs_coef
       if (JV > 64) throw std::runtime_error("projection against more than 64 vectors");
       k::mdot<T>(N, (int)JV, D(BV), N, D(w), W->dsm, W->dpart, S());
-      k::gemv_dev<T>(N, (int)JV, T(-1), D(V), N, W->dsm, T(1), D(w), S(), y ? W->hsm + kCoef : nullptr);
+      k::gemv_dev<T>(N, (int)JV, -1.0, D(V), N, W->dsm, 1.0, D(w), S(), y ? W->hsm + kCoef : nullptr);
       return;
     }
     // up to 63 columns: a pass leaves its coefficients on the device between
@@ -254,7 +254,7 @@ template <class T> struct DevJd {
           first = false;
         } else {
           gemvc(N, (int)JV, BV, N, w, y + JV);
-          gemvn(N, (int)JV, H(-1), V, N, y + JV, H(1), w);
+          gemvn(N, (int)JV, -1.0, V, N, y + JV, 1.0, w);
           nrn = nrm2(N, w);
         }
         if (nrnd)

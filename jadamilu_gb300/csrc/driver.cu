@@ -939,15 +939,15 @@ template <class T> struct PjdRun {
     if (which == 1 || which == 3) k::spmv<T>(g.A, jd.D(x), jd.D(y), g.W.st);
     if ((which == 1 || which == 4) && gep) k::spmv<T>(g.Bm, jd.D(x), jd.D(by), g.W.st);
   }
-  void builtin_mv_shift(long x, long y, long yb, typename HostOf<T>::type a) {
+  void builtin_mv_shift(long x, long y, long yb, double a) {
     g.n_matvec++;
-    k::spmv_shift<T>(g.A, gep ? &g.Bm : nullptr, todev(a), jd.D(x), jd.D(y), jd.D(yb), g.W.st);
+    k::spmv_shift<T>(g.A, gep ? &g.Bm : nullptr, a, jd.D(x), jd.D(y), jd.D(yb), g.W.st);
   }
-  int builtin_inner(int cols, long U, long BU, long z, long r, long p, typename HostOf<T>::type eta, bool first,
+  int builtin_inner(int cols, long U, long BU, long z, long r, long p, double eta, bool first,
                     bool posdef, T* rho, const T* rho0) {
     g.n_matvec++;
     return k::inner_one<T>(g.A, gep ? &g.Bm : nullptr, cols, jd.D(U), jd.D(BU), jd.D(z), jd.D(r), jd.D(p),
-                           todev(eta), first, posdef, rho, rho0, g.W.hsm + DevJd<T>::kScal,
+                           eta, first, posdef, rho, rho0, g.W.hsm + DevJd<T>::kScal,
                            g.W.dpart + k::kPartialHead, g.W.hpart, g.W.dbar, g.W.one, g.W.st);
   }
   void precond(long rhs, long sol);
@@ -1172,9 +1172,9 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
   jd.precond = [&R](long r, long s) { R.precond(r, s); };
   jd.device_ops = !user_mv && g_opt.fuse_inner != 0;
   if (jd.device_ops)
-    jd.matvec_shift = [&R](long x, long y, long yb, typename HostOf<T>::type a) { R.builtin_mv_shift(x, y, yb, a); };
+    jd.matvec_shift = [&R](long x, long y, long yb, double a) { R.builtin_mv_shift(x, y, yb, a); };
   if (jd.device_ops)
-    jd.inner_one = [&R](int k, long U, long BU, long z, long r, long p, typename HostOf<T>::type eta,
+    jd.inner_one = [&R](int k, long U, long BU, long z, long r, long p, double eta,
                         bool first, bool posdef, T* rho, const T* rho0) {
       return R.builtin_inner(k, U, BU, z, r, p, eta, first, posdef, rho, rho0);
     };

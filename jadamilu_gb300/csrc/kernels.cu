@@ -128,10 +128,18 @@ template <class T> void spmv(const SellMatrix<T>& A, const T* x, T* y, cudaStrea
   COUNT_LAUNCH();
 }
 // -------------------------------------------------------------- BLAS-1 ----
+// Complex vectors times real scalars: the products with a zero imaginary part,
+// which cannot change a sum, are left out.  FP64 instructions are the bound of
+// the complex kernels from about 1e5 rows on (2 FMA per SM and cycle).
+__device__ __forceinline__ double axpy_re(double a, double x, double y) { return fma(a, x, y); }
+__device__ __forceinline__ zc axpy_re(double a, zc x, zc y) { return zc(fma(a, x.x, y.x), fma(a, x.y, y.y)); }
+__device__ __forceinline__ double im_(double) { return 0.0; }
+__device__ __forceinline__ double im_(zc a) { return a.y; }
 template <class T> __global__ void axpy_kernel(long n, T a, const T* __restrict__ x, T* __restrict__ y) {
   pdl_begin();
+  const bool real = im_(a) == 0.0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    y[i] = fma_(a, x[i], y[i]);
+    y[i] = real ? axpy_re(rl(a), x[i], y[i]) : fma_(a, x[i], y[i]);
 }
 template <class T> __global__ void scal_kernel(long n, double a, T* x) {
   pdl_begin();
@@ -167,8 +175,9 @@ __device__ __forceinline__ zc ldcg_(const zc* p) {
   return zc(v.x, v.y);
 }
 
-constexpr int MD_CH = 8;       // columns per group (one grid row of CTAs)
-constexpr int MD_GROUPS = 16;  // column groups of one call: k <= 128
+constexpr int MD_CH = 8;       // most columns that one tree carries
+constexpr int MD_GROUPS = 32;  // column groups of one call
+constexpr int MD_COLS = 128;   // columns of one call
 constexpr int MD_WARPS = TPB / 32;
 // Long vectors: up to two rows per thread, enough CTAs in flight to stream V
 // at full bandwidth.  Vectors under 4096 rows keep one CTA per 2048 rows, the
@@ -185,7 +194,7 @@ static inline int md_grid(long n) {
 constexpr int MD_HEAD = MD_GROUPS * (int)sizeof(unsigned);
 static_assert(MD_HEAD <= kPartialHead * (int)sizeof(double), "the counters fit before the partials");
 long mdot_partial_size(long n, int k) {
-  return (long)md_grid(n) * ((k + MD_CH - 1) / MD_CH) * MD_CH + kPartialHead;
+  return (long)md_grid(n) * k + kPartialHead;
 }
 
 // The warp tree (lane pairs 16, 8, 4, 2, 1 apart) of CH values per lane (CH a
@@ -210,8 +219,9 @@ template <class T, int CH> __device__ __forceinline__ T md_tree(T (&v)[CH], int 
   return v[0];
 }
 template <int CH> __device__ __forceinline__ int md_col(int lane) {
-  static_assert(CH == 1 || CH == 2 || CH == 8, "column groups of 1, 2 or 8");
-  return CH == 1 ? 0 : CH == 2 ? (lane >> 4) & 1 : ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+  static_assert(CH == 1 || CH == 2 || CH == 4 || CH == 8, "column groups of 1, 2, 4 or 8");
+  const int b4 = (lane >> 4) & 1, b3 = (lane >> 3) & 1, b2 = (lane >> 2) & 1;
+  return CH == 1 ? 0 : CH == 2 ? b4 : CH == 4 ? b4 * 2 + b3 : b4 * 4 + b3 * 2 + b2;
 }
 
 // The sum of one column's g partials by one warp, in the order of TPB threads
@@ -286,6 +296,13 @@ __device__ __forceinline__ bool md_finish(T (&acc)[CH], int nc, int c0, unsigned
   return true;
 }
 
+// Columns per group of mdot: four instead of eight leave registers for more
+// resident CTAs, which hide the trees.  us for 25 columns, eight -> four
+// (GB300): n = 1e6 136 -> 96.6, 262144 42.3 -> 32.5, 64000 13.5 -> 11.6, complex
+// 262144 105 -> 76.2; for five columns at n = 64000 8.0 -> 9.9.
+constexpr int MD_GRP = 4;
+static_assert(MD_COLS <= MD_GRP * MD_GROUPS, "a counter for every group");
+
 // V^H w in one launch, a grid row of CTAs per group of CH columns.
 // xcol, when given, is column k - 1 (a vector that does not follow V's others).
 template <class T, int CH>
@@ -325,13 +342,14 @@ __global__ void __launch_bounds__(TPB) mdot_kernel(long n, int k, const T* __res
 template <class T>
 void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s, const T* xcol) {
   if (k <= 0) return;
-  if (k > MD_CH * MD_GROUPS) throw std::runtime_error("mdot: too many columns");
+  if (k > MD_COLS) throw std::runtime_error("mdot: too many columns");
   unsigned char* buf = reinterpret_cast<unsigned char*>(partial);
   const int g = md_grid(n);
   if (k == 1)
     launch_k(mdot_kernel<T, 1>, dim3(g), dim3(TPB), 0, s, n, k, V, ldv, w, xcol, buf, out);
   else
-    launch_k(mdot_kernel<T, MD_CH>, dim3(g, (k + MD_CH - 1) / MD_CH), dim3(TPB), 0, s, n, k, V, ldv, w, xcol, buf, out);
+    launch_k(mdot_kernel<T, MD_GRP>, dim3(g, (k + MD_GRP - 1) / MD_GRP), dim3(TPB), 0, s, n, k, V, ldv, w, xcol,
+             buf, out);
   g_launches += 1;
 }
 
@@ -340,8 +358,8 @@ constexpr int GMV_MAX = 64;
 template <class T> struct SmallVec { T v[GMV_MAX]; };
 
 template <class T>
-__global__ void __launch_bounds__(TPB) jd_basis_gemv_dev_kernel(long n, int k, T alpha, const T* __restrict__ V, long ldv,
-                                                       const T* __restrict__ y, T beta, T* __restrict__ w,
+__global__ void __launch_bounds__(TPB) jd_basis_gemv_dev_kernel(long n, int k, double alpha, const T* __restrict__ V, long ldv,
+                                                       const T* __restrict__ y, double beta, T* __restrict__ w,
                                                        T* __restrict__ hy) {
   pdl_begin();
   __shared__ T ys[GMV_MAX];
@@ -353,27 +371,27 @@ __global__ void __launch_bounds__(TPB) jd_basis_gemv_dev_kernel(long n, int k, T
   for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
     T acc = T(0);
     for (int c = 0; c < k; ++c) acc = fma_(V[i + (long)c * ldv], ys[c], acc);
-    T o = (beta == T(0)) ? T(0) : beta * w[i];
-    w[i] = fma_(alpha, acc, o);
+    const T o = beta == 0 ? T(0) : beta == 1 ? w[i] : beta * w[i];
+    w[i] = axpy_re(alpha, acc, o);
   }
 }
 template <class T>
-__global__ void __launch_bounds__(TPB) jd_basis_gemv_val_kernel(long n, int k, T alpha, const T* __restrict__ V, long ldv,
-                                                       SmallVec<T> y, T beta, T* __restrict__ w) {
+__global__ void __launch_bounds__(TPB) jd_basis_gemv_val_kernel(long n, int k, double alpha, const T* __restrict__ V, long ldv,
+                                                       SmallVec<T> y, double beta, T* __restrict__ w) {
   pdl_begin();
   for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
     T acc = T(0);
     for (int c = 0; c < k; ++c) acc = fma_(V[i + (long)c * ldv], y.v[c], acc);
-    T o = (beta == T(0)) ? T(0) : beta * w[i];
-    w[i] = fma_(alpha, acc, o);
+    const T o = beta == 0 ? T(0) : beta == 1 ? w[i] : beta * w[i];
+    w[i] = axpy_re(alpha, acc, o);
   }
 }
 template <class T>
-void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, T* w, cudaStream_t s, T* hy) {
+void gemv_dev(long n, int k, double alpha, const T* V, long ldv, const T* y, double beta, T* w, cudaStream_t s, T* hy) {
   if (k > GMV_MAX) throw std::runtime_error("gemv_dev: too many columns");
   if (k <= 0) {
-    if (!(beta == T(1))) {
-      if (beta == T(0)) fill(n, T(0), w, s);
+    if (beta != 1) {
+      if (beta == 0) fill(n, T(0), w, s);
       else throw std::runtime_error("gemv_dev: unsupported beta");
     }
     return;
@@ -382,10 +400,10 @@ void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, 
   COUNT_LAUNCH();
 }
 template <class T>
-void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* yh, T beta, T* w, cudaStream_t s) {
+void gemv_val(long n, int k, double alpha, const T* V, long ldv, const T* yh, double beta, T* w, cudaStream_t s) {
   if (k > GMV_MAX) throw std::runtime_error("gemv_val: too many columns");
   if (k <= 0) {
-    if (beta == T(0)) fill(n, T(0), w, s);
+    if (beta == 0) fill(n, T(0), w, s);
     return;
   }
   SmallVec<T> y;
@@ -394,24 +412,9 @@ void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* yh, T beta,
   COUNT_LAUNCH();
 }
 
-// the real part of acc + conj(a) b, with the roundings of fma_, and a real
-// scalar's a x + y (the products with its zero imaginary part left out)
+// the real part of acc + conj(a) b, with the roundings of fma_
 __device__ __forceinline__ double dot_re(double a, double b, double acc) { return fma(a, b, acc); }
 __device__ __forceinline__ double dot_re(zc a, zc b, double acc) { return fma(a.x, b.x, fma(a.y, b.y, acc)); }
-__device__ __forceinline__ double axpy_re(double a, double x, double y) { return fma(a, x, y); }
-__device__ __forceinline__ zc axpy_re(double a, zc x, zc y) { return zc(fma(a, x.x, y.x), fma(a, x.y, y.y)); }
-
-// ------------------------------------------- the inner iteration, fused ----
-// One CG / sQMR iteration outside the preconditioner is a chain of vector
-// updates with an inner product after each.  Every launch of the chain costs
-// about as much as its bytes up to n = 1e5, and an update's result is read
-// back by the inner product that follows, so an update kernel also accumulates
-// that product over the rows it writes, in the row order and with the tail
-// (md_finish) of mdot: the roundings are those of separate kernels.  Scalars
-// stay in device memory (results of earlier kernels of the chain); the last
-// kernel puts them into pinned host memory itself.  Against ten kernels and a
-// copy (GB300, per solve): Anderson 16^3 (n = 4096) 16 % less, Laplacian 20^3
-// 51.6 -> 46.8 ms, tight-binding 64^3 (n = 262144, complex) 406 -> 389 ms.
 
 // w = w - V y (y in device memory), out[0] = x^H w (x = nullptr: w^H w); then,
 // with nsc > 0, the nsc scalars from sc on go to the host's pinned hsc.  ratio,
@@ -439,7 +442,7 @@ __global__ void __launch_bounds__(TPB) gemv_dot_kernel(long n, int k, const T* _
       a0 = fma_(V[i + (long)c * ldv], ys[c], a0);
       a1 = fma_(V[i1 + (long)c * ldv], ys[c], a1);
     }
-    const T r0 = fma_(T(-1), a0, o0), r1 = fma_(T(-1), a1, o1);
+    const T r0 = o0 - a0, r1 = o1 - a1;
     w[i] = r0;
     dot[0] = fma_(cj(x ? x0 : r0), r0, dot[0]);
     if (two) {
@@ -495,7 +498,7 @@ template <class T, bool GEP>
 __global__ void __launch_bounds__(TPB) spmv_shift_kernel(int n, const int64_t* __restrict__ sptr,
                                                          const int* __restrict__ col, const T* __restrict__ val,
                                                          const int64_t* __restrict__ bptr, const int* __restrict__ bcol,
-                                                         const T* __restrict__ bval, T a, const T* __restrict__ x,
+                                                         const T* __restrict__ bval, double a, const T* __restrict__ x,
                                                          T* __restrict__ y, T* __restrict__ yb) {
   pdl_launch();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -515,10 +518,10 @@ __global__ void __launch_bounds__(TPB) spmv_shift_kernel(int n, const int64_t* _
     for (int64_t q = b2 + lane + kSellPre * 32; q < e2; q += 32) u = fma_(bval[q], x[__ldg(bcol + q)], u);
     yb[r] = u;
   }
-  y[r] = fma_(a, u, acc);
+  y[r] = axpy_re(a, u, acc);
 }
 template <class T>
-void spmv_shift(const SellMatrix<T>& A, const SellMatrix<T>* B, T a, const T* x, T* y, T* yb, cudaStream_t s) {
+void spmv_shift(const SellMatrix<T>& A, const SellMatrix<T>* B, double a, const T* x, T* y, T* yb, cudaStream_t s) {
   const int64_t* bp = B ? B->sptr : nullptr;
   const int* bc = B ? B->col : nullptr;
   const T* bv = B ? B->val : nullptr;
@@ -542,7 +545,7 @@ __global__ void __launch_bounds__(TPB) cg_residual_kernel(long n, const double* 
   for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
     const T t = axpy_re(a, q[i], r[i]);
     r[i] = t;
-    dot[0] = fma_(cj(t), t, dot[0]);
+    dot[0] = T(dot_re(t, t, rl(dot[0])));
   }
   if (!md_finish<T, 1>(dot, 1, 0, buf, out)) return;
   __syncthreads();
@@ -560,23 +563,23 @@ void cg_residual(long n, const double* al, const T* q, T* r, T* out, const T* sc
 // its first iteration: x2 = s p, x = x2); with B also bt += al bp.  The first
 // iteration's x and bt start from zero.
 template <class T, bool SMOOTH, bool FIRST>
-__global__ void __launch_bounds__(TPB) cg_iterate_kernel(long n, T a, double s, const T* __restrict__ p,
-                                                         T* __restrict__ x2, T* __restrict__ x, T al,
+__global__ void __launch_bounds__(TPB) cg_iterate_kernel(long n, double a, double s, const T* __restrict__ p,
+                                                         T* __restrict__ x2, T* __restrict__ x, double al,
                                                          const T* __restrict__ bp, T* __restrict__ bt) {
   pdl_begin();
   for (long i = blockIdx.x * (long)TPB + threadIdx.x; i < n; i += (long)gridDim.x * TPB) {
     if (SMOOTH) {
-      const T t = FIRST ? s * p[i] : s * fma_(a, p[i], x2[i]);
+      const T t = FIRST ? s * p[i] : s * axpy_re(a, p[i], x2[i]);
       x2[i] = t;
-      x[i] = FIRST ? t : fma_(T(1), t, x[i]);
+      x[i] = FIRST ? t : x[i] + t;
     } else {
-      x[i] = fma_(a, p[i], FIRST ? T(0) : x[i]);
+      x[i] = axpy_re(a, p[i], FIRST ? T(0) : x[i]);
     }
-    if (bt) bt[i] = fma_(al, bp[i], FIRST ? T(0) : bt[i]);
+    if (bt) bt[i] = axpy_re(al, bp[i], FIRST ? T(0) : bt[i]);
   }
 }
 template <class T>
-void cg_iterate(long n, bool smooth, bool first, T a, double sc, const T* p, T* x2, T* x, T al, const T* bp, T* bt,
+void cg_iterate(long n, bool smooth, bool first, double a, double sc, const T* p, T* x2, T* x, double al, const T* bp, T* bt,
                 cudaStream_t s) {
   auto go = [&](auto kern) { launch_k(kern, dim3(grid_1d(n)), dim3(TPB), 0, s, n, a, sc, p, x2, x, al, bp, bt); };
   if (smooth && first) go(cg_iterate_kernel<T, true, true>);
@@ -592,7 +595,7 @@ void cg_iterate(long n, bool smooth, bool first, T a, double sc, const T* p, T* 
 // the norm, with their roundings.
 template <class T, bool GEP>
 __global__ void __launch_bounds__(TPB) ritz_kernel(long n, int k, const T* __restrict__ V, const T* __restrict__ Wv,
-                                                   const T* __restrict__ B, long ld, SmallVec<T> y, T a,
+                                                   const T* __restrict__ B, long ld, SmallVec<T> y, double a,
                                                    T* __restrict__ u, T* __restrict__ r, T* __restrict__ bu,
                                                    unsigned char* buf, T* out) {
   pdl_begin();
@@ -616,14 +619,14 @@ __global__ void __launch_bounds__(TPB) ritz_kernel(long n, int k, const T* __res
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       if (q == 1 && i + step >= n) break;
-      T ub = fma_(T(1), su[q], T(0));
+      T ub = su[q];
       u[at[q]] = ub;
       if (GEP) {
-        ub = fma_(T(1), sb[q], T(0));
+        ub = sb[q];
         bu[at[q]] = ub;
         dot[GEP] = fma_(cj(ub), ub, dot[GEP]);
       }
-      const T t = fma_(a, ub, fma_(T(1), sr[q], T(0)));
+      const T t = axpy_re(a, ub, sr[q]);
       r[at[q]] = t;
       dot[0] = fma_(cj(t), t, dot[0]);
     }
@@ -631,7 +634,7 @@ __global__ void __launch_bounds__(TPB) ritz_kernel(long n, int k, const T* __res
   md_finish<T, GEP ? 2 : 1>(dot, GEP ? 2 : 1, 0, buf, out);
 }
 template <class T>
-void ritz(long n, int k, const T* V, const T* Wv, const T* B, long ld, const T* yh, T a, T* u, T* r, T* bu, T* out,
+void ritz(long n, int k, const T* V, const T* Wv, const T* B, long ld, const T* yh, double a, T* u, T* r, T* bu, T* out,
           T* partial, cudaStream_t s) {
   if (k < 1 || k > GMV_MAX) throw std::runtime_error("ritz: bad column count");
   SmallVec<T> y;
@@ -733,7 +736,7 @@ template <class T> struct InnerOne {
   const int64_t *sptr, *bptr;   // A and, for GEP, B
   const int *col, *bcol;
   const T *val, *bval;
-  T eta;                        // q = A p + eta (B) p
+  double eta;                   // q = A p + eta (B) p
   bool first, posdef;
   T *rho, *hsc;
   const T* rho0;                // the previous iteration's rho (not read in the first)
@@ -810,19 +813,26 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
     z[j] = r[j] = p[j] = q[j] = T(0);
     if (has(j)) z[j] = a.z[row0 + j * step];
   }
-  for (int c0 = 0; c0 < a.k; c0 += MD_CH) {
-    const int nc = min(MD_CH, a.k - c0);
-    T acc[MD_CH];
+  auto project = [&](auto ch, int c0) {
+    constexpr int CH = decltype(ch)::value;
+    const int nc = min(CH, a.k - c0);
+    T acc[CH];
 #pragma unroll
-    for (int c = 0; c < MD_CH; ++c) acc[c] = T(0);
+    for (int c = 0; c < CH; ++c) acc[c] = T(0);
 #pragma unroll
     for (int j = 0; j < RM; ++j)
       if (has(j)) {
 #pragma unroll
-        for (int c = 0; c < MD_CH; ++c)
+        for (int c = 0; c < CH; ++c)
           if (c < nc) acc[c] = fma_(cj(a.BU[row0 + j * step + (long)(c0 + c) * n]), z[j], acc[c]);
       }
     put(acc, nc, pa + (long)c0 * g);
+  };
+  for (int c0 = 0; c0 < a.k;) {  // a tree no wider than the columns left
+    const int left = a.k - c0;
+    if (left == 1) project(std::integral_constant<int, 1>(), c0++);
+    else if (left <= 4 || sizeof(T) == 16) project(std::integral_constant<int, 4>(), c0), c0 += 4;
+    else project(std::integral_constant<int, MD_CH>(), c0), c0 += MD_CH;
   }
 #pragma unroll
   for (int j = 0; j < RM; ++j)
@@ -852,7 +862,7 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
 #pragma unroll
     for (int j = 0; j < RM; ++j)
       if (has(j)) {
-        z[j] = fma_(T(-1), acc[j], z[j]);
+        z[j] = z[j] - acc[j];
         dot[0] = dot_re(r[j], z[j], dot[0]);
       }
     put(dot, 1, pb);
@@ -909,7 +919,7 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
           u = sell_row(fb, qb + kSellPre * 32, eb, a.bcol, a.bval, (const T*)a.p);
           a.z[i] = u;
         }
-        q[j] = fma_(a.eta, u, acc);
+        q[j] = axpy_re(a.eta, u, acc);
         dot[0] = fma_(cj(a.U[i]), q[j], dot[0]);
         if (GEP) dot[GEP] = fma_(cj(a.BU[i]), q[j], dot[GEP]);
       }
@@ -928,7 +938,7 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
 #pragma unroll
     for (int j = 0; j < RM; ++j)
       if (has(j)) {
-        q[j] = fma_(T(-1), fma_(a.BU[row0 + j * step], uq, T(0)), q[j]);
+        q[j] = q[j] - fma_(a.BU[row0 + j * step], uq, T(0));
         dot[0] = dot_re(p[j], q[j], dot[0]);
       }
     put(dot, 1, pd);
@@ -1055,7 +1065,7 @@ template <class T> static int one_pick(long n, bool gep) {
 }
 template <class T> bool inner_one_ok(long n, int k, bool gep) { return k <= kOneMaxCols && one_pick<T>(n, gep) >= 0; }
 template <class T>
-int inner_one(const SellMatrix<T>& A, const SellMatrix<T>* B, int k, const T* U, const T* BU, T* z, T* r, T* p, T eta,
+int inner_one(const SellMatrix<T>& A, const SellMatrix<T>* B, int k, const T* U, const T* BU, T* z, T* r, T* p, double eta,
               bool first, bool posdef, T* rho, const T* rho0, T* hsc, T* part, double* hpart, unsigned* bar, OneState& st,
               cudaStream_t s) {
   InnerOne<T> a;
@@ -1978,18 +1988,18 @@ template <class T, class S> void ildl_apply_graph(DevFactor<S>& F, bool spd, con
   template void gemv_dot<T>(long, int, const T*, long, const T*, T*, const T*, T*, T*, cudaStream_t, const T*, int, \
                             T*, const T*, const T*, double*);                                     \
   template bool inner_one_ok<T>(long, int, bool);                                                 \
-  template int inner_one<T>(const SellMatrix<T>&, const SellMatrix<T>*, int, const T*, const T*, T*, T*, T*, T, bool, \
+  template int inner_one<T>(const SellMatrix<T>&, const SellMatrix<T>*, int, const T*, const T*, T*, T*, T*, double, bool, \
                             bool, T*, const T*, T*, T*, double*, unsigned*, OneState&, cudaStream_t); \
   template void cg_direction<T>(long, const T*, const double*, bool, T*, T*, cudaStream_t);           \
-  template void spmv_shift<T>(const SellMatrix<T>&, const SellMatrix<T>*, T, const T*, T*, T*, cudaStream_t); \
+  template void spmv_shift<T>(const SellMatrix<T>&, const SellMatrix<T>*, double, const T*, T*, T*, cudaStream_t); \
   template void cg_residual<T>(long, const double*, const T*, T*, T*, const T*, int, T*, T*, cudaStream_t); \
-  template void cg_iterate<T>(long, bool, bool, T, double, const T*, T*, T*, T, const T*, T*, cudaStream_t); \
+  template void cg_iterate<T>(long, bool, bool, double, double, const T*, T*, T*, double, const T*, T*, cudaStream_t); \
   template void scal<T>(long, double, T*, cudaStream_t);                                           \
   template void fill<T>(long, T, T*, cudaStream_t);                                                \
   template void mdot<T>(long, int, const T*, long, const T*, T*, T*, cudaStream_t, const T*);      \
-  template void gemv_dev<T>(long, int, T, const T*, long, const T*, T, T*, cudaStream_t, T*);      \
-  template void ritz<T>(long, int, const T*, const T*, const T*, long, const T*, T, T*, T*, T*, T*, T*, cudaStream_t); \
-  template void gemv_val<T>(long, int, T, const T*, long, const T*, T, T*, cudaStream_t);          \
+  template void gemv_dev<T>(long, int, double, const T*, long, const T*, double, T*, cudaStream_t, T*);      \
+  template void ritz<T>(long, int, const T*, const T*, const T*, long, const T*, double, T*, T*, T*, T*, T*, cudaStream_t); \
+  template void gemv_val<T>(long, int, double, const T*, long, const T*, double, T*, cudaStream_t);          \
   template void rmult<T>(long, int, int, const T*, long, const T*, T*, cudaStream_t);              \
   template void diagsolve<T>(long, const double*, const T*, T*, cudaStream_t);
 JD_INST_T(double)

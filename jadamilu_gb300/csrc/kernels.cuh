@@ -120,18 +120,18 @@ template <class T> void fill(long n, T v, T* x, cudaStream_t s);
 // out[c] = V(:,c)^H w for c < k (deterministic reduction), the last column
 // being xcol when that is given; out may be pinned host memory; partial needs
 // mdot_partial_size(n,k) entries
-constexpr int kPartialHead = 8;  // entries before the partials: the arrival counters
+constexpr int kPartialHead = 16;  // entries before the partials: the arrival counters
 long mdot_partial_size(long n, int k);
 template <class T>
 void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s, const T* xcol = nullptr);
-// w = beta*w + alpha*V*y, y (k <= 64 entries) in device memory (copied to the
+// w = beta*w + alpha*V*y (alpha and beta real), y (k <= 64 entries) in device memory (copied to the
 // pinned hy when that is given) or by value
 template <class T>
-void gemv_dev(long n, int k, T alpha, const T* V, long ldv, const T* y, T beta, T* w, cudaStream_t s, T* hy = nullptr);
-template <class T> void gemv_val(long n, int k, T alpha, const T* V, long ldv, const T* y_host, T beta, T* w, cudaStream_t s);
+void gemv_dev(long n, int k, double alpha, const T* V, long ldv, const T* y, double beta, T* w, cudaStream_t s, T* hy = nullptr);
+template <class T> void gemv_val(long n, int k, double alpha, const T* V, long ldv, const T* y_host, double beta, T* w, cudaStream_t s);
 // u = V y, r = W y + a bu (bu = u, or B y), out[0] = r^H r (with B: out[1] = bu^H bu), y on the host
 template <class T>
-void ritz(long n, int k, const T* V, const T* Wv, const T* B, long ld, const T* yh, T a, T* u, T* r, T* bu, T* out,
+void ritz(long n, int k, const T* V, const T* Wv, const T* B, long ld, const T* yh, double a, T* u, T* r, T* bu, T* out,
           T* partial, cudaStream_t s);
 // The kernels of one fused CG / sQMR iteration (kernels.cu); partial as for mdot.
 // w -= V y (y in device memory, 1 <= k <= 64), *out = x^H w (x null: w^H w), then
@@ -145,7 +145,7 @@ template <class T>
 void cg_direction(long n, const T* rho, const double* be, bool posdef, T* p, T* z, cudaStream_t s);
 // y = A x + a x; with B: yb = B x, y = A x + a yb
 template <class T>
-void spmv_shift(const SellMatrix<T>& A, const SellMatrix<T>* B, T a, const T* x, T* y, T* yb, cudaStream_t s);
+void spmv_shift(const SellMatrix<T>& A, const SellMatrix<T>* B, double a, const T* x, T* y, T* yb, cudaStream_t s);
 // r -= *al q, *out = r^H r, then hsc[0..nsc) = sc[0..nsc) (hsc: pinned host memory)
 template <class T>
 void cg_residual(long n, const double* al, const T* q, T* r, T* out, const T* sc, int nsc, T* hsc, T* partial,
@@ -164,13 +164,13 @@ int inner_one_partials(long n, int k);
 constexpr int kMaxPartials = 152 * 8;  // most CTAs of a reduction
 double md_sum_host(const double* p, int g);
 template <class T>
-int inner_one(const SellMatrix<T>& A, const SellMatrix<T>* B, int k, const T* U, const T* BU, T* z, T* r, T* p, T eta,
+int inner_one(const SellMatrix<T>& A, const SellMatrix<T>* B, int k, const T* U, const T* BU, T* z, T* r, T* p, double eta,
               bool first, bool posdef, T* rho, const T* rho0, T* hsc, T* part, double* hpart, unsigned* bar, OneState& st,
               cudaStream_t s);
 // smooth: x2 = sc (x2 + a p), x += x2 (first: x2 = sc p, x = x2); else x += a p (first: from zero); bt, when given,
 // += al bp (first: from zero)
 template <class T>
-void cg_iterate(long n, bool smooth, bool first, T a, double sc, const T* p, T* x2, T* x, T al, const T* bp, T* bt,
+void cg_iterate(long n, bool smooth, bool first, double a, double sc, const T* p, T* x2, T* x, double al, const T* bp, T* bt,
                 cudaStream_t s);
 // out(:,c) = V * Q(:,c), c < keep, Q K x K column-major (host values)
 template <class T> void rmult(long n, int K, int keep, const T* V, long ldv, const T* Q_host, T* out, cudaStream_t s);
