@@ -35,8 +35,46 @@ static double wall() {
 }
 
 // --------------------------------------------------------- device matrix ----
+// device buffer for the caller's triangle while a matrix is built from it
+struct SellStage {
+  void* p = nullptr;
+  int64_t cap = 0;
+  void* need(int64_t bytes) {
+    if (bytes > cap) {
+      release();
+      CK(cudaMalloc(&p, bytes));
+      cap = bytes;
+    }
+    return p;
+  }
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    cap = 0;
+  }
+};
+template <class T> void sell_slices(SellMatrix<T>& M, int ns) {
+  if (ns <= M.cap_slices) return;
+  if (M.sptr) cudaFree(M.sptr);
+  M.sptr = nullptr;
+  M.cap_slices = 0;
+  CK(cudaMalloc(&M.sptr, sizeof(int64_t) * (ns + 1)));
+  M.cap_slices = ns;
+}
+template <class T> void sell_slots(SellMatrix<T>& M, int64_t slots) {
+  if (slots <= M.cap_slots) return;
+  if (M.col) cudaFree(M.col);
+  if (M.val) cudaFree(M.val);
+  M.col = nullptr;
+  M.val = nullptr;
+  M.cap_slots = 0;
+  CK(cudaMalloc(&M.col, sizeof(int) * slots));
+  CK(cudaMalloc(&M.val, sizeof(T) * slots));
+  M.cap_slots = slots;
+}
+// The host pass: for matrices with a row beyond what the device build takes.
 template <class T, class H>
-void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, cudaStream_t st) {
+void build_sell_host(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, cudaStream_t st) {
   std::vector<int> cnt(n, 0);
   for (int i = 0; i < n; ++i)
     for (int p = ia[i] - 1; p < ia[i + 1] - 1; ++p) {
@@ -85,21 +123,52 @@ void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& 
       }
     }
   }
-  if (M.sptr) { cudaFree(M.sptr); cudaFree(M.col); cudaFree(M.val); }
-  M.n = n;
-  M.nslices = ns;
+  sell_slices(M, ns);
+  sell_slots(M, std::max<int64_t>(1, sp[ns]));
   M.nnz = rp[n];
   M.stored = sp[ns];
-  CK(cudaMalloc(&M.sptr, sizeof(int64_t) * (ns + 1)));
-  CK(cudaMalloc(&M.col, sizeof(int) * std::max<int64_t>(1, sp[ns])));
-  CK(cudaMalloc(&M.val, sizeof(T) * std::max<int64_t>(1, sp[ns])));
   CK(cudaMemcpyAsync(M.sptr, sp.data(), sizeof(int64_t) * (ns + 1), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(M.col, scol.data(), sizeof(int) * sp[ns], cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(M.val, sval.data(), sizeof(T) * sp[ns], cudaMemcpyHostToDevice, st));
   CK(cudaStreamSynchronize(st));
 }
+// The matrix for the products from the caller's triangle; keep: a staging
+// buffer that outlives the call (a solver's), else one of its own.
+template <class T, class H>
+void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, cudaStream_t st,
+                SellStage* keep = nullptr) {
+  static_assert(sizeof(T) == sizeof(H), "the values are copied as they are");
+  const int64_t nnz = (int64_t)ia[n] - 1;
+  if (nnz < 0) throw std::runtime_error("row pointers out of range");
+  struct Own : SellStage {
+    ~Own() { release(); }
+  } own;
+  SellStage& stage = keep ? *keep : own;
+  const int ns = (n + 31) / 32;
+  sell_slices(M, ns);
+  unsigned long long info[4] = {};
+  const bool built = k::sell_from_triangle<T>(
+      n, ia, ja, a, stage.need(k::sell_work_bytes(n, nnz, sizeof(T))), M.sptr, info,
+      [&](int64_t slots, int** col, T** val) {
+        sell_slots(M, std::max<int64_t>(1, slots));
+        *col = M.col;
+        *val = M.val;
+      },
+      st);
+  if (built) {
+    M.stored = (int64_t)info[0];
+    M.nnz = (int64_t)info[1];
+    if (!keep) CK(cudaStreamSynchronize(st));  // the staging buffer goes
+  } else {
+    build_sell_host<T>(n, ia, ja, a, M, st);
+  }
+  M.n = n;
+  M.nslices = ns;
+}
 template <class T> void free_sell(SellMatrix<T>& M) {
-  if (M.sptr) { cudaFree(M.sptr); cudaFree(M.col); cudaFree(M.val); }
+  void* ps[] = {M.sptr, M.col, M.val};
+  for (void* p : ps)
+    if (p) cudaFree(p);
   M = SellMatrix<T>();
 }
 
@@ -627,6 +696,7 @@ template <class T> struct Global {
   DevFactor<B> Fb;         // device factor, bfloat16 storage
   double* ddiag = nullptr; // diagonal preconditioner on the device
   SellMatrix<T> A, Bm;     // built-in matvec operands
+  SellStage stage;         // and the buffer they are built from
   bool resident = false;   // A (and B) prepared on the device by the caller
   int nfactor = 0;
   double t_factor = 0, t_upload = 0;
@@ -645,6 +715,7 @@ template <class T> struct Global {
     cleanup1();
     free_sell(A);
     free_sell(Bm);
+    stage.release();
     resident = false;
     W.release();
   }
@@ -1141,8 +1212,8 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
   // operands of the built-in matvec
   if (!user_mv && !g.resident) {
     if (ja[0] < 0) throw std::runtime_error("diagonal preconditioning needs the reverse-communication matvec");
-    build_sell<T>(n, ia, ja, a, g.A, g.W.st);
-    if (gep) build_sell<T>(n, ib, jb, b, g.Bm, g.W.st);
+    build_sell<T>(n, ia, ja, a, g.A, g.W.st, &g.stage);
+    if (gep) build_sell<T>(n, ib, jb, b, g.Bm, g.W.st, &g.stage);
   }
   // initial guesses
   if (NINIT > 0)
@@ -1903,7 +1974,7 @@ JDG_API int jdgpu_dprepare_matrix(int n, const int* ia, const int* ja, const dou
   try {
     Global<double>& g = G<double>();
     g.W.ensure(n, n);
-    build_sell<double>(n, ia, ja, a, g.A, g.W.st);
+    build_sell<double>(n, ia, ja, a, g.A, g.W.st, &g.stage);
     g.resident = true;
     return 0;
   } catch (std::exception& e) {

@@ -1,6 +1,7 @@
 // Launch wrappers for the sm_103a kernels of the Jacobi-Davidson hot path.
 // Every wrapper enqueues on the given stream and never synchronises.
 #pragma once
+#include <functional>
 #include <vector>
 
 #include "common.cuh"
@@ -16,6 +17,7 @@ template <class T> struct SellMatrix {
   int64_t* sptr = nullptr;
   int* col = nullptr;
   T* val = nullptr;
+  int64_t cap_slices = 0, cap_slots = 0;  // what sptr and col / val have room for
 };
 
 // A block of consecutive rows [s0, s0 + m) after the bulk levels.  Forward:
@@ -113,6 +115,16 @@ void add_launches(long long n);
 // device flag that a kernel sets when a bounded wait inside it ran out
 int* wait_expired_flag();
 
+// SELL-32 of the full Hermitian matrix from the caller's host CSR of one triangle (1-based; a: n values of T's
+// layout).  work: sell_work_bytes(n, nnz, sizeof(T)) device bytes; sptr: (n + 31) / 32 + 1 entries; info_host: 4
+// entries, then stored slots and full nonzeros in the first two; room: called once, after a synchronisation, with the
+// slots needed, gives the col and val arrays.  False (nothing built): a row too long for it, use the host pass.  The
+// host arrays are read before it returns.
+int64_t sell_work_bytes(int n, int64_t nnz, int64_t value);
+template <class T>
+bool sell_from_triangle(int n, const int* ia, const int* ja, const void* a, void* work, int64_t* sptr,
+                        unsigned long long* info_host, const std::function<void(int64_t, int**, T**)>& room,
+                        cudaStream_t s);
 template <class T> void spmv(const SellMatrix<T>& A, const T* x, T* y, cudaStream_t s);
 template <class T> void axpy(long n, T a, const T* x, T* y, cudaStream_t s);
 template <class T> void scal(long n, double a, T* x, cudaStream_t s);
