@@ -269,6 +269,9 @@ JDG_API int jdgpu_dildl_apply_noalloc(int n, const int* ia, const int* ja, const
  * -1 on bad arguments, -99 on a CUDA error. */
 JDG_API int jdgpu_deig_grad(int n, const int* ia, const int* ja, int neig, const double* X, int ldx,
                             const double* w, const double* bdiag, double* grad);
+/* The same with X row by row: n x neig, row-major without padding. */
+JDG_API int jdgpu_deig_grad_rows(int n, const int* ia, const int* ja, int neig, const double* X, const double* w,
+                                 const double* bdiag, double* grad);
 
 /* Gradient of a loss L(x) of one eigenvector with respect to every stored
  * entry of A: x an eigenvector of A x = lambda B x (B = I, or diagonal with

@@ -70,6 +70,7 @@ def load(build_if_missing: bool = True):
     L.jdgpu_revcom_device_ptr.argtypes = [C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p)]
     L.jdgpu_revcom_device_ptr.restype = C.c_int
     L.jdgpu_deig_grad.argtypes = [C.c_int, _P, _P, C.c_int, _P, C.c_int, _P, _P, _P]
+    L.jdgpu_deig_grad_rows.argtypes = [C.c_int, _P, _P, C.c_int, _P, _P, _P, _P]
     L.jdgpu_dildl_bench.argtypes = [C.c_int, _P, _P, _P, C.c_double, C.c_double, C.c_double, C.c_int, C.c_int,
                                     C.c_int, _P]
     L.jdgpu_dprepare_matrix.argtypes = [C.c_int, _P, _P, _P]
@@ -372,12 +373,17 @@ def eig_grad(A, X, w=None, bdiag=None):
     _require_gpu(L)
     a, ja, ia = _matrix(A, np.float64)
     n = len(ia) - 1
-    X = np.asfortranarray(np.asarray(X, np.float64).reshape(n, -1))
+    X = np.asarray(X, np.float64).reshape(n, -1)
+    by_column = X.flags.f_contiguous
+    X = X if by_column else np.ascontiguousarray(X)
     k = X.shape[1]
     w = np.ones(k) if w is None else np.ascontiguousarray(w, np.float64)
     bd = None if bdiag is None else np.ascontiguousarray(bdiag, np.float64)
     g = np.zeros(len(a))
-    r = L.jdgpu_deig_grad(n, _p(ia), _p(ja), k, _p(X), n, _p(w), _p(bd) if bd is not None else None, _p(g))
+    if by_column:
+        r = L.jdgpu_deig_grad(n, _p(ia), _p(ja), k, _p(X), n, _p(w), _p(bd) if bd is not None else None, _p(g))
+    else:
+        r = L.jdgpu_deig_grad_rows(n, _p(ia), _p(ja), k, _p(X), _p(w), _p(bd) if bd is not None else None, _p(g))
     if r != 0:
         raise RuntimeError(f"jdgpu_deig_grad failed ({r})")
     return g

@@ -8,9 +8,15 @@
 // the weighted sum over the eigenpairs; for a cluster of equal eigenvalues it
 // is basis-independent when the whole cluster is included with one weight.
 //
-// Device work: per-column normalisation s_k = x_k^T B x_k (B diagonal or I)
-// by a deterministic two-pass reduction, then one pass over the nonzeros
-// (thread per row, rows read their entries and the eigenvector rows once).
+// Device work: per-column normalisation s_k = x_k^T B x_k (B diagonal or I) by
+// a deterministic reduction, then one pass over the nonzeros (thread per row,
+// rows read their entries and the eigenvector rows once).  X may come column by
+// column or row by row: the kernels read either, so no caller has to transpose.
+//
+// Bound: the copies from and to the caller's arrays (28 MB at n = 260100 and
+// six pairs, 0.2 ms at 150 GB/s) and one allocation.  Nine allocations, a column at
+// a time in the normalisation and a transposition of C-order eigenvectors on
+// the host made it 2.8 ms a call, now 0.63 ms (GB300).
 #include <algorithm>
 #include <vector>
 
@@ -23,53 +29,138 @@ namespace {
 
 constexpr int GR_TPB = 256;
 constexpr int GR_MAXK = 64;
+constexpr int GR_CH = 8;  // columns a thread carries at once
 
-// partial[b * k + c] = sum over this block's rows of bdiag_i * x_c(i)^2
-__global__ void colnorm_partial_kernel(int n, int k, const double* __restrict__ X, long ldx,
-                                       const double* __restrict__ bdiag, double* __restrict__ partial) {
-  __shared__ double red[GR_TPB];
-  for (int c = 0; c < k; ++c) {
-    double s = 0;
-    for (int i = blockIdx.x * GR_TPB + threadIdx.x; i < n; i += gridDim.x * GR_TPB) {
-      const double v = X[(long)c * ldx + i];
-      s += (bdiag ? bdiag[i] : 1.0) * v * v;
+// coef[c] = w_c / sum_i bdiag_i x_c(i)^2; X(i, c) at i * rs + c * cs.  Every CTA
+// writes its partial sums, the last to arrive (count starts at zero) adds them
+// in CTA order: strided over 32 lanes, then the warp tree.
+__global__ void __launch_bounds__(GR_TPB) colnorm_kernel(int n, int k, const double* __restrict__ X, long rs, long cs,
+                                                         const double* __restrict__ bdiag,
+                                                         const double* __restrict__ w, double* partial,
+                                                         unsigned* count, double* __restrict__ coef) {
+  __shared__ double red[GR_TPB / 32][GR_CH];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nb = gridDim.x;
+  for (int c0 = 0; c0 < k; c0 += GR_CH) {
+    double s[GR_CH] = {};
+    for (int i = blockIdx.x * GR_TPB + threadIdx.x; i < n; i += nb * GR_TPB) {
+      const double b = bdiag ? bdiag[i] : 1.0;
+#pragma unroll
+      for (int c = 0; c < GR_CH; ++c)
+        if (c0 + c < k) {
+          const double v = X[i * rs + (c0 + c) * cs];
+          s[c] += b * v * v;
+        }
     }
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = GR_TPB / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-      __syncthreads();
+#pragma unroll
+    for (int c = 0; c < GR_CH; ++c) {
+      for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+      if (lane == 0) red[wid][c] = s[c];
     }
-    if (threadIdx.x == 0) partial[(long)blockIdx.x * k + c] = red[0];
     __syncthreads();
+    if (threadIdx.x < GR_CH && c0 + threadIdx.x < k) {
+      double t = 0;
+      for (int q = 0; q < GR_TPB / 32; ++q) t += red[q][threadIdx.x];
+      partial[(long)(c0 + threadIdx.x) * nb + blockIdx.x] = t;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(count, 1u) == (unsigned)nb - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  for (int c = wid; c < k; c += GR_TPB / 32) {
+    double t = 0;
+    for (int b = lane; b < nb; b += 32) t += __ldcg(partial + (long)c * nb + b);
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) coef[c] = w[c] / t;
   }
 }
 
-// coef[c] = w_c / sum_b partial[b * k + c]  (fixed order)
-__global__ void colnorm_final_kernel(int nb, int k, const double* __restrict__ partial, const double* __restrict__ w,
-                                     double* __restrict__ coef) {
-  const int c = threadIdx.x;
-  if (c >= k) return;
-  double s = 0;
-  for (int b = 0; b < nb; ++b) s += partial[(long)b * k + c];
-  coef[c] = w[c] / s;
-}
-
-// grad[q] = c_q * sum_c coef_c x_c(i) x_c(j), i the row of stored entry q
-__global__ void eig_grad_kernel(int n, int k, const int* __restrict__ ia, const int* __restrict__ ja,
-                                const double* __restrict__ X, long ldx, const double* __restrict__ coef,
-                                double* __restrict__ grad) {
+// grad[q] = c_q * sum_c coef_c x_c(i) x_c(j), i the row of stored entry q; KM
+// columns in registers.  A row pointer or column out of range sets *bad.
+template <int KM>
+__global__ void __launch_bounds__(GR_TPB) eig_grad_kernel(int n, int nnz, int k, const int* __restrict__ ia,
+                                                          const int* __restrict__ ja, const double* __restrict__ X,
+                                                          long rs, long cs, const double* __restrict__ coef,
+                                                          double* __restrict__ grad, unsigned* bad) {
   const int i = blockIdx.x * GR_TPB + threadIdx.x;
   if (i >= n) return;
-  double xi[GR_MAXK];
-  for (int c = 0; c < k; ++c) xi[c] = coef[c] * X[(long)c * ldx + i];
+  double xi[KM];
+#pragma unroll
+  for (int c = 0; c < KM; ++c) xi[c] = c < k ? coef[c] * X[i * rs + c * cs] : 0.0;
   const int b = ia[i] - 1, e = ia[i + 1] - 1;
+  if (b < 0 || e > nnz) {
+    *bad = 1;
+    return;
+  }
   for (int q = b; q < e; ++q) {
     const int j = ja[q] - 1;
+    if (j < 0 || j >= n) {
+      *bad = 1;
+      continue;
+    }
     double g = 0;
-    for (int c = 0; c < k; ++c) g += xi[c] * X[(long)c * ldx + j];
+#pragma unroll
+    for (int c = 0; c < KM; ++c)
+      if (c < k) g += xi[c] * X[j * rs + c * cs];
     grad[q] = (j == i) ? g : 2.0 * g;
   }
+}
+
+int eig_grad(int n, const int* ia, const int* ja, int neig, const double* X, long rs, long cs, long xlen,
+             const double* w, const double* bdiag, double* grad) {
+  const int nnz = ia[n] - 1;
+  if (nnz < 0) return -1;
+  unsigned char* base = nullptr;
+  int rc = 0;
+  try {
+    const int nb = std::min(std::max(1, (n + GR_TPB - 1) / GR_TPB), 152 * 4);
+    size_t used = 0;
+    auto place = [&](size_t bytes) {
+      const size_t at = used;
+      used += (bytes + 255) / 256 * 256;
+      return at;
+    };
+    const size_t oia = place(sizeof(int) * ((size_t)n + 1)), oja = place(sizeof(int) * (size_t)std::max(1, nnz)),
+                 oX = place(sizeof(double) * (size_t)xlen), ow = place(sizeof(double) * neig),
+                 ob = place(bdiag ? sizeof(double) * (size_t)n : 0), op = place(sizeof(double) * (size_t)nb * neig),
+                 oc = place(sizeof(double) * neig), of = place(2 * sizeof(unsigned)),
+                 og = place(sizeof(double) * (size_t)std::max(1, nnz));
+    CK(cudaMalloc(&base, used));
+    int *dia = (int*)(base + oia), *dja = (int*)(base + oja);
+    double *dX = (double*)(base + oX), *dw = (double*)(base + ow), *db = bdiag ? (double*)(base + ob) : nullptr,
+           *dpart = (double*)(base + op), *dcoef = (double*)(base + oc), *dg = (double*)(base + og);
+    unsigned* flags = (unsigned*)(base + of);  // arrival counter, out-of-range flag
+    const cudaStream_t st = nullptr;
+    CK(cudaMemsetAsync(flags, 0, 2 * sizeof(unsigned), st));
+    CK(cudaMemcpyAsync(dX, X, sizeof(double) * (size_t)xlen, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(dw, w, sizeof(double) * neig, cudaMemcpyHostToDevice, st));
+    if (bdiag) CK(cudaMemcpyAsync(db, bdiag, sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    colnorm_kernel<<<nb, GR_TPB, 0, st>>>(n, neig, dX, rs, cs, db, dw, dpart, flags, dcoef);
+    CK(cudaMemcpyAsync(dia, ia, sizeof(int) * ((size_t)n + 1), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(dja, ja, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice, st));
+    const dim3 g((n + GR_TPB - 1) / GR_TPB);
+    auto go = [&](auto kern) { kern<<<g, GR_TPB, 0, st>>>(n, nnz, neig, dia, dja, dX, rs, cs, dcoef, dg, flags + 1); };
+    if (neig <= 8) go(eig_grad_kernel<8>);
+    else if (neig <= 16) go(eig_grad_kernel<16>);
+    else go(eig_grad_kernel<GR_MAXK>);
+    CK(cudaGetLastError());
+    k::add_launches(2);
+    unsigned bad = 0;
+    CK(cudaMemcpyAsync(&bad, flags + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(grad, dg, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (bad) rc = -1;
+  } catch (std::exception& e) {
+    std::fprintf(stderr, "jdgpu_deig_grad: %s\n", e.what());
+    rc = -99;
+  }
+  cudaFree(base);
+  return rc;
 }
 
 }  // namespace
@@ -82,42 +173,10 @@ using namespace jdg;
 JDG_API int jdgpu_deig_grad(int n, const int* ia, const int* ja, int neig, const double* X, int ldx,
                             const double* w, const double* bdiag, double* grad) {
   if (n <= 0 || neig <= 0 || neig > GR_MAXK || ldx < n) return -1;
-  const int nnz = ia[n] - 1;
-  int *dia = nullptr, *dja = nullptr;
-  double *dX = nullptr, *dw = nullptr, *db = nullptr, *dpart = nullptr, *dcoef = nullptr, *dg = nullptr;
-  int rc = 0;
-  try {
-    const int nb = std::min(std::max(1, (n + GR_TPB - 1) / GR_TPB), 152 * 4);
-    CK(cudaMalloc(&dia, sizeof(int) * (n + 1)));
-    CK(cudaMalloc(&dja, sizeof(int) * std::max(1, nnz)));
-    CK(cudaMalloc(&dX, sizeof(double) * (size_t)ldx * neig));
-    CK(cudaMalloc(&dw, sizeof(double) * neig));
-    CK(cudaMalloc(&dpart, sizeof(double) * (size_t)nb * neig));
-    CK(cudaMalloc(&dcoef, sizeof(double) * neig));
-    CK(cudaMalloc(&dg, sizeof(double) * std::max(1, nnz)));
-    if (bdiag) CK(cudaMalloc(&db, sizeof(double) * n));
-    CK(cudaMemcpy(dia, ia, sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dja, ja, sizeof(int) * nnz, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dX, X, sizeof(double) * (size_t)ldx * neig, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dw, w, sizeof(double) * neig, cudaMemcpyHostToDevice));
-    if (bdiag) CK(cudaMemcpy(db, bdiag, sizeof(double) * n, cudaMemcpyHostToDevice));
-    colnorm_partial_kernel<<<nb, GR_TPB>>>(n, neig, dX, ldx, db, dpart);
-    colnorm_final_kernel<<<1, GR_MAXK>>>(nb, neig, dpart, dw, dcoef);
-    eig_grad_kernel<<<(n + GR_TPB - 1) / GR_TPB, GR_TPB>>>(n, neig, dia, dja, dX, ldx, dcoef, dg);
-    CK(cudaGetLastError());
-    k::add_launches(3);
-    CK(cudaMemcpy(grad, dg, sizeof(double) * nnz, cudaMemcpyDeviceToHost));
-  } catch (std::exception& e) {
-    std::fprintf(stderr, "jdgpu_deig_grad: %s\n", e.what());
-    rc = -99;
-  }
-  cudaFree(dia);
-  cudaFree(dja);
-  cudaFree(dX);
-  cudaFree(dw);
-  cudaFree(db);
-  cudaFree(dpart);
-  cudaFree(dcoef);
-  cudaFree(dg);
-  return rc;
+  return eig_grad(n, ia, ja, neig, X, 1, ldx, (long)ldx * (neig - 1) + n, w, bdiag, grad);
+}
+JDG_API int jdgpu_deig_grad_rows(int n, const int* ia, const int* ja, int neig, const double* X, const double* w,
+                                 const double* bdiag, double* grad) {
+  if (n <= 0 || neig <= 0 || neig > GR_MAXK) return -1;
+  return eig_grad(n, ia, ja, neig, X, neig, 1, (long)n * neig, w, bdiag, grad);
 }
