@@ -2329,21 +2329,24 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
     upload_factor(F, D, st);
     const size_t vb = sizeof(double) * n;
     enum { X, BX, G, R1, R2, Y, V, W, W1, W2, MU, T1, T2, BD, NV };
-    std::vector<double*> vec(NV, nullptr);
-    for (int k = 0; k < NV; ++k) CK(cudaMalloc(&vec[k], vb));
-    double *dsm, *dpart;
-    CK(cudaMalloc(&dsm, sizeof(double) * 4));
-    CK(cudaMalloc(&dpart, sizeof(double) * k::mdot_partial_size(n, 1)));
-    CK(cudaMemset(dpart, 0, sizeof(double) * k::mdot_partial_size(n, 1)));
+    // one allocation: the vectors, the scalars and the reduction's partials
+    const size_t vs = (vb + 255) / 256 * 256, ps = sizeof(double) * k::mdot_partial_size(n, 1);
+    unsigned char* base = nullptr;
+    CK(cudaMalloc(&base, vs * NV + 256 + ps));
+    std::vector<double*> vec(NV);
+    for (int k = 0; k < NV; ++k) vec[k] = (double*)(base + vs * k);
+    double* const dsm = (double*)(base + vs * NV);
+    double* const dpart = (double*)(base + vs * NV + 256);
+    double* hsm = nullptr;
+    CK(cudaMallocHost(&hsm, sizeof(double) * 8));
+    CK(cudaMemsetAsync(dpart, 0, ps, st));
     CK(cudaMemcpyAsync(vec[X], xin, vb, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(vec[G], g, vb, cudaMemcpyHostToDevice, st));
     if (bdiag) CK(cudaMemcpyAsync(vec[BD], bdiag, vb, cudaMemcpyHostToDevice, st));
     auto dot = [&](const double* u, const double* w) {
-      double h = 0;
-      k::mdot<double>(n, 1, u, n, w, dsm, dpart, st);
-      CK(cudaMemcpyAsync(&h, dsm, sizeof(double), cudaMemcpyDeviceToHost, st));
+      k::mdot<double>(n, 1, u, n, w, hsm, dpart, st);
       CK(cudaStreamSynchronize(st));
-      return h;
+      return hsm[0];
     };
     auto bmul = [&](const double* u, double* w) {  // w = B u
       if (bdiag) k::diagsolve<double>(n, vec[BD], u, w, st);
@@ -2355,13 +2358,16 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
     if (!(xbx > 0)) throw std::runtime_error("x^T B x is not positive");
     k::scal<double>(n, 1 / std::sqrt(xbx), vec[X], st);
     k::scal<double>(n, 1 / std::sqrt(xbx), vec[BX], st);
+    // The projections leave their coefficient on the device, and alfa stays
+    // there until r2^T y is known: one synchronisation per iteration.
+    enum { COEF, ALFA, BETA2 };
     auto proj_t = [&](double* u) {  // u := P^T u = u - B x (x^T u)
-      const double c = dot(vec[X], u);
-      k::axpy<double>(n, -c, vec[BX], u, st);
+      k::mdot<double>(n, 1, vec[X], n, u, dsm + COEF, dpart, st);
+      k::axpy_dev<double>(n, dsm + COEF, 1.0, vec[BX], u, st);
     };
     auto proj = [&](double* u) {  // u := P u = u - x (x^T B u)
-      const double c = dot(vec[BX], u);
-      k::axpy<double>(n, -c, vec[X], u, st);
+      k::mdot<double>(n, 1, vec[BX], n, u, dsm + COEF, dpart, st);
+      k::axpy_dev<double>(n, dsm + COEF, 1.0, vec[X], u, st);
     };
     auto op = [&](const double* u, double* w) {  // w = P^T (A - lambda B) P u
       CK(cudaMemcpyAsync(vec[T1], u, vb, cudaMemcpyDeviceToDevice, st));
@@ -2371,18 +2377,21 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
       k::axpy<double>(n, -lambda, vec[T2], w, st);
       proj_t(w);
     };
-    auto prec = [&](const double* u, double* w) {  // w = P |F|^{-1} P^T u
+    // w = P |F|^{-1} P^T u; returns u^T w
+    auto prec = [&](const double* u, double* w) {
       CK(cudaMemcpyAsync(vec[T1], u, vb, cudaMemcpyDeviceToDevice, st));
       proj_t(vec[T1]);
       k::ildl_apply<double, double>(D, true, vec[T1], w, st);
       proj(w);
+      k::mdot<double>(n, 1, u, n, w, hsm + BETA2, dpart, st);
+      CK(cudaStreamSynchronize(st));
+      return hsm[BETA2];
     };
     // preconditioned MINRES from mu = 0 on b = P^T g
     CK(cudaMemcpyAsync(vec[R1], vec[G], vb, cudaMemcpyDeviceToDevice, st));
     proj_t(vec[R1]);
     CK(cudaMemcpyAsync(vec[R2], vec[R1], vb, cudaMemcpyDeviceToDevice, st));
-    prec(vec[R1], vec[Y]);
-    double beta1 = dot(vec[R1], vec[Y]);
+    double beta1 = prec(vec[R1], vec[Y]);
     if (beta1 < 0) throw std::runtime_error("the preconditioner is not positive definite");
     beta1 = std::sqrt(beta1);
     for (int k2 : {W, W1, W2, MU}) k::fill<double>(n, 0.0, vec[k2], st);
@@ -2395,13 +2404,13 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
       k::scal<double>(n, 1 / beta, vec[V], st);
       op(vec[V], vec[Y]);
       if (it >= 2) k::axpy<double>(n, -beta / oldb, vec[R1], vec[Y], st);
-      const double alfa = dot(vec[V], vec[Y]);
-      k::axpy<double>(n, -alfa / beta, vec[R2], vec[Y], st);
+      k::mdot<double>(n, 1, vec[V], n, vec[Y], dsm + ALFA, dpart, st);
+      CK(cudaMemcpyAsync(hsm + ALFA, dsm + ALFA, sizeof(double), cudaMemcpyDeviceToHost, st));
+      k::axpy_dev<double>(n, dsm + ALFA, beta, vec[R2], vec[Y], st);
       std::swap(vec[R1], vec[R2]);
       CK(cudaMemcpyAsync(vec[R2], vec[Y], vb, cudaMemcpyDeviceToDevice, st));
-      prec(vec[R2], vec[Y]);
+      const double bb = prec(vec[R2], vec[Y]), alfa = hsm[ALFA];
       oldb = beta;
-      const double bb = dot(vec[R2], vec[Y]);
       if (bb < 0) throw std::runtime_error("the preconditioner is not positive definite");
       beta = std::sqrt(bb);
       const double oldeps = epsln, delta = cs * dbar + sn * alfa, gbar = sn * dbar - cs * alfa;
@@ -2437,9 +2446,8 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
       out[0] = it;
       out[1] = beta1 > 0 ? rnorm / beta1 : 0;
     }
-    for (auto* v : vec) cudaFree(v);
-    cudaFree(dsm);
-    cudaFree(dpart);
+    cudaFree(base);
+    cudaFreeHost(hsm);
     free_factor(D);
     free_sell(Am);
     cudaStreamDestroy(st);

@@ -319,6 +319,14 @@ template <class T> __global__ void axpy_kernel(long n, T a, const T* __restrict_
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     y[i] = real ? axpy_re(rl(a), x[i], y[i]) : fma_(a, x[i], y[i]);
 }
+// y -= (Re *c / den) x with *c in device memory (the result of an earlier reduction)
+template <class T>
+__global__ void axpy_dev_kernel(long n, const T* c, double den, const T* __restrict__ x, T* __restrict__ y) {
+  pdl_begin();
+  const double a = den == 1 ? -rl(*c) : -rl(*c) / den;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    y[i] = axpy_re(a, x[i], y[i]);
+}
 template <class T> __global__ void scal_kernel(long n, double a, T* x) {
   pdl_begin();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) x[i] = a * x[i];
@@ -330,6 +338,9 @@ template <class T> __global__ void fill_kernel(long n, T v, T* x) {
 static inline int grid_1d(long n) { return (int)std::min<long>(nblk(n), 152L * 16); }
 template <class T> void axpy(long n, T a, const T* x, T* y, cudaStream_t s) {
   if (n > 0) { launch_k(axpy_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, a, x, y); COUNT_LAUNCH(); }
+}
+template <class T> void axpy_dev(long n, const T* c, double den, const T* x, T* y, cudaStream_t s) {
+  if (n > 0) { launch_k(axpy_dev_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, c, den, x, y); COUNT_LAUNCH(); }
 }
 template <class T> void scal(long n, double a, T* x, cudaStream_t s) {
   if (n > 0) { launch_k(scal_kernel<T>, dim3(grid_1d(n)), dim3(TPB), 0, s, n, a, x); COUNT_LAUNCH(); }
@@ -2174,6 +2185,7 @@ template <class T, class S> void ildl_apply_graph(DevFactor<S>& F, bool spd, con
   template void spmv_shift<T>(const SellMatrix<T>&, const SellMatrix<T>*, double, const T*, T*, T*, cudaStream_t); \
   template void cg_residual<T>(long, const double*, const T*, T*, T*, const T*, int, T*, T*, cudaStream_t); \
   template void cg_iterate<T>(long, bool, bool, double, double, const T*, T*, T*, double, const T*, T*, cudaStream_t); \
+  template void axpy_dev<T>(long, const T*, double, const T*, T*, cudaStream_t);                  \
   template void scal<T>(long, double, T*, cudaStream_t);                                           \
   template void fill<T>(long, T, T*, cudaStream_t);                                                \
   template void mdot<T>(long, int, const T*, long, const T*, T*, T*, cudaStream_t, const T*);      \

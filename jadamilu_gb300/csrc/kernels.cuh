@@ -127,6 +127,8 @@ bool sell_from_triangle(int n, const int* ia, const int* ja, const void* a, void
                         cudaStream_t s);
 template <class T> void spmv(const SellMatrix<T>& A, const T* x, T* y, cudaStream_t s);
 template <class T> void axpy(long n, T a, const T* x, T* y, cudaStream_t s);
+// y -= (Re *c / den) x with *c in device memory
+template <class T> void axpy_dev(long n, const T* c, double den, const T* x, T* y, cudaStream_t s);
 template <class T> void scal(long n, double a, T* x, cudaStream_t s);
 template <class T> void fill(long n, T v, T* x, cudaStream_t s);
 // out[c] = V(:,c)^H w for c < k (deterministic reduction), the last column
