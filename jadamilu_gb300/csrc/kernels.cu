@@ -413,43 +413,36 @@ template <int CH> __device__ __forceinline__ int md_col(int lane) {
   return CH == 1 ? 0 : CH == 2 ? b4 : CH == 4 ? b4 * 2 + b3 : b4 * 4 + b3 * 2 + b2;
 }
 
-// The sum of one column's g partials by one warp, in the order of TPB threads
-// striding over them (32 w + lane, step TPB, for w = 0 .. 7), the warp tree of
-// each w, then w in order (up to 32 partials only w = 0 holds any); every lane
-// returns it.  A dependent float64 addition takes some 50 cycles here, so the
-// shorter chain counts.
-template <class T> __device__ __forceinline__ T md_sum_partials(const T* p, int g, int lane) {
-  if (g <= 32) {
-    T s[1] = {T(0)};
-    if (lane < g) s[0] += ldcg_(p + lane);
-    return md_tree(s, lane);
-  }
-  T s[MD_WARPS];
+// A lane's share of the g partials of nc columns: those at 32 w + lane, step
+// TPB, of warp w.  The warp tree of each w, then w in order, completes the sum.
+template <class T, int CH>
+__device__ __forceinline__ T (*md_partials(const T* p, int nc, int g, int w, int lane, T (&s)[CH]))[CH] {
 #pragma unroll
-  for (int w = 0; w < MD_WARPS; ++w) s[w] = T(0);
-  for (int q0 = 0; q0 < g; q0 += TPB)
+  for (int c = 0; c < CH; ++c) s[c] = T(0);
+#pragma unroll 1
+  for (int q = 32 * w + lane; q < g; q += TPB)
 #pragma unroll
-    for (int w = 0; w < MD_WARPS; ++w) {
-      const int q = q0 + 32 * w + lane;
-      if (q < g) s[w] += ldcg_(p + q);
-    }
-  const T t8 = md_tree(s, lane);  // the sum of stride w in lane 4 * bit-reversed w
-  T t = T(0);
-#pragma unroll
-  for (int w = 0; w < MD_WARPS; ++w)
-    t += shfl_idx_any(t8, ((w >> 2) & 1) * 16 + ((w >> 1) & 1) * 8 + (w & 1) * 4);
-  return t;
+    for (int c = 0; c < CH; ++c)
+      if (c < nc) s[c] += ldcg_(p + (long)c * g + q);
+  return &s;
+}
+
+// The sum of one column's g <= 32 partials by one warp; every lane returns it.
+template <class T> __device__ __forceinline__ T md_sum_32(const T* p, int g, int lane) {
+  T s[1] = {T(0)};
+  if (lane < g) s[0] += ldcg_(p + lane);
+  return md_tree(s, lane);
 }
 
 // The end of a reduction whose threads hold CH partial sums each: a column's
 // sums go up the warp tree, then over the CTA's warps in order; the CTA of the
-// group that arrives last (a counter, no waiting) adds the CTAs' partials, one
-// warp per column.  The order is that of TPB threads striding over the g
-// partials (32 s + lane, step TPB, for s = 0 .. 7), the warp tree of each s,
-// then s in order, so the result does not depend on which CTA is last.  This
-// tail bounds the short reductions: one CTA going through the columns one by
-// one with two barriers each took 12 to 50 us a call (n = 8000: 12.1 us with
-// 25 columns at most), and the groups finish side by side.
+// group that arrives last (a counter, no waiting) adds the CTAs' partials the
+// same way, its threads striding over them, so the result does not depend on
+// which CTA is last.  This tail bounds the short reductions (store, fence,
+// atomic, loads, and two chains of dependent float64 additions of some 50
+// cycles each).  us a call (GB300), one CTA going through the columns one by
+// one with two barriers each -> here: one column n = 4096 4.9 -> 4.1, 64000 7.3
+// -> 6.9, 1e6 14.9 -> 12.5; 12 to 50 us on average over the solves before.
 // Returns true in the CTA that wrote the group's results.
 template <class T, int CH>
 __device__ __forceinline__ bool md_finish(T (&acc)[CH], int nc, int c0, unsigned char* buf, T* out) {
@@ -477,9 +470,22 @@ __device__ __forceinline__ bool md_finish(T (&acc)[CH], int nc, int c0, unsigned
   }
   __syncthreads();
   if (!last) return false;
-  if (wid < nc) {
-    const T t = md_sum_partials(partial + (long)(c0 + wid) * g, g, lane);
-    if (lane == 0) out[c0 + wid] = t;
+  if (g <= 32) {  // only warp 0 would find partials: a warp per column, and done
+    if (wid < nc) {
+      const T t = md_sum_32(partial + (long)(c0 + wid) * g, g, lane);
+      if (lane == 0) out[c0 + wid] = t;
+    }
+  } else {
+    T s[CH];
+    const T f = md_tree(*md_partials<T, CH>(partial + (long)c0 * g, nc, g, wid, lane, s), lane);
+    if (lane % (32 / CH) == 0) red[wid][md_col<CH>(lane)] = f;
+    __syncthreads();
+    if (threadIdx.x < nc) {
+      T t = T(0);
+#pragma unroll
+      for (int q = 0; q < MD_WARPS; ++q) t += red[q][threadIdx.x];
+      out[c0 + threadIdx.x] = t;
+    }
   }
   if (threadIdx.x == 0) *count = 0u;
   return true;
@@ -544,6 +550,7 @@ void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, c
 
 // ------------------------------------------------------ V y (tall-skinny) ----
 constexpr int GMV_MAX = 64;
+constexpr int kColBatch = 4;  // columns of a projection whose loads are in flight at once
 template <class T> struct SmallVec { T v[GMV_MAX]; };
 
 template <class T>
@@ -626,10 +633,25 @@ __global__ void __launch_bounds__(TPB) gemv_dot_kernel(long n, int k, const T* _
     const long i1 = two ? i + step : i;
     const T o0 = w[i], o1 = w[i1], x0 = x ? x[i] : T(0), x1 = x ? x[i1] : T(0);
     T a0 = T(0), a1 = T(0);
-#pragma unroll 4
-    for (int c = 0; c < k; ++c) {
-      a0 = fma_(V[i + (long)c * ldv], ys[c], a0);
-      a1 = fma_(V[i1 + (long)c * ldv], ys[c], a1);
+    int c0 = 0;
+    for (; c0 + kColBatch <= k; c0 += kColBatch) {  // the loads of a batch first, then its products in order
+      T v0[kColBatch], v1[kColBatch];
+#pragma unroll
+      for (int c = 0; c < kColBatch; ++c) {
+        v0[c] = V[i + (long)(c0 + c) * ldv];
+        v1[c] = V[i1 + (long)(c0 + c) * ldv];
+      }
+#pragma unroll
+      for (int c = 0; c < kColBatch; ++c) {
+        a0 = fma_(v0[c], ys[c0 + c], a0);
+        a1 = fma_(v1[c], ys[c0 + c], a1);
+      }
+    }
+#pragma unroll 1
+    for (; c0 < k; ++c0) {
+      const T v0 = V[i + (long)c0 * ldv], v1 = V[i1 + (long)c0 * ldv];
+      a0 = fma_(v0, ys[c0], a0);
+      a1 = fma_(v1, ys[c0], a1);
     }
     const T r0 = o0 - a0, r1 = o1 - a1;
     w[i] = r0;
@@ -648,8 +670,11 @@ template <class T>
 void gemv_dot(long n, int k, const T* V, long ldv, const T* y, T* w, const T* x, T* out, T* partial, cudaStream_t s,
               const T* sc, int nsc, T* hsc, const T* rnum, const T* rden, double* ratio) {
   if (k < 1 || k > GMV_MAX) throw std::runtime_error("projection against more than 64 vectors");
-  launch_k(gemv_dot_kernel<T>, dim3(md_grid(n)), dim3(TPB), 0, s, n, k, V, ldv, y, w, x,
-           reinterpret_cast<unsigned char*>(partial), out, sc, nsc, hsc, rnum, rden, ratio);
+  auto go = [&](auto kern) {
+    launch_k(kern, dim3(md_grid(n)), dim3(TPB), 0, s, n, k, V, ldv, y, w, x, reinterpret_cast<unsigned char*>(partial), out,
+             sc, nsc, hsc, rnum, rden, ratio);
+  };
+  go(gemv_dot_kernel<T>);
   COUNT_LAUNCH();
 }
 
@@ -891,8 +916,8 @@ int* wait_expired_flag() {
 // Bound: the chain of six phases, each a barrier, a few L2 latencies (0.14 us)
 // and dependent float64 additions (some 50 cycles each), and from 1e5 rows on
 // the FP64 units (2 FMA per SM and cycle).  us per iteration with 5 columns,
-// separate kernels -> one (GB300): n = 4096 28.6 -> 20.5, 15625 30.2 -> 24.6,
-// 64000 45.0 -> 28.7, 262144 65.0 -> 53.3, complex 262144 122 -> 110.
+// separate kernels -> one (GB300): n = 4096 26.5 -> 20.5, 15625 29.8 -> 24.6,
+// 64000 46.8 -> 26.7, 262144 59.3 -> 50.3, complex 262144 109 -> 102.
 constexpr int kOneMaxCols = GMV_MAX;
 constexpr int kBarPolls = 1 << 22;
 int inner_one_partials(long n, int k) { return md_grid(n) * (k + 3); }
@@ -959,10 +984,10 @@ constexpr int kOneRows = 2;  // rows of a thread (mdot's grid gives it that many
 template <class T, bool GEP, int VC, bool CLU>
 __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_constant__ InnerOne<T> a) {
   __shared__ T red[VC][MD_WARPS][MD_CH];
-  __shared__ T ys[kOneMaxCols];
+  __shared__ T ys[kOneMaxCols + 4 * VC];
   __shared__ double sc[2];
   const int vc = threadIdx.x / TPB, vt = threadIdx.x % TPB, vb = blockIdx.x * VC + vc;
-  const int lane = threadIdx.x & 31, vw = vt >> 5, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, vw = vt >> 5;
   constexpr int RM = kOneRows;
   const bool on = vb < a.g;
   const int n = a.n, g = a.g, step = g * TPB, row0 = vb * TPB + vt;
@@ -990,6 +1015,35 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
       dst[(long)vt * g + vb] = t;
     }
     __syncthreads();
+  };
+  // sums over the grid of nc <= 4 columns' partials p, in md_finish's order, by this virtual CTA's warps; the caller
+  // synchronises before it reads dst
+  auto total = [&](const auto* p, int nc, auto* dst) {
+    using E = std::remove_const_t<std::remove_reference_t<decltype(*p)>>;
+    if (g <= 32) {
+      if (vw < nc) {
+        const E t = md_sum_32(p + (long)vw * g, g, lane);
+        if (lane == 0) dst[vw] = t;
+      }
+      return;
+    }
+    E* rd = reinterpret_cast<E*>(&red[vc][0][0]);
+    if (nc == 1) {
+      E s[1];
+      const E v = md_tree(*md_partials<E, 1>(p, nc, g, vw, lane, s), lane);
+      if (lane == 0) rd[vw * 4] = v;
+    } else if (nc > 0) {
+      E s[4];
+      const E v = md_tree(*md_partials<E, 4>(p, nc, g, vw, lane, s), lane);
+      if (lane % 8 == 0) rd[vw * 4 + md_col<4>(lane)] = v;
+    }
+    __syncthreads();
+    if (vt < nc) {
+      E t = E(0);
+#pragma unroll
+      for (int q = 0; q < MD_WARPS; ++q) t += rd[q * 4 + vt];
+      dst[vt] = t;
+    }
   };
   T* pa = a.part;                                          // BU^H z
   double* pb = reinterpret_cast<double*>(pa + (long)a.k * g);  // Re r^H z
@@ -1031,11 +1085,11 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
     }
   if (!barrier()) return;
   // 2: z -= U c, rho = r^H z
-  for (int c = wid; c < a.k; c += MD_WARPS * VC) {
-    const T t = md_sum_partials(pa + (long)c * g, g, lane);
-    if (lane == 0) ys[c] = t;
+  for (int c0 = 0; c0 < a.k; c0 += 4 * VC) {
+    const int c = c0 + 4 * vc;
+    total(pa + (long)c * g, min(4, max(0, a.k - c)), ys + c);
+    __syncthreads();
   }
-  __syncthreads();
   {
     double dot[1] = {0.0};
     T acc[RM];
@@ -1058,13 +1112,8 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
   }
   if (!barrier()) return;
   // 3: the search direction
-  if (wid == 0) {
-    const double t = md_sum_partials((const double*)pb, g, lane);
-    if (lane == 0) {
-      sc[0] = t;
-      sc[1] = a.first ? 0.0 : t / rl(*a.rho0);
-    }
-  }
+  total((const double*)pb, vc == 0 ? 1 : 0, sc);
+  if (threadIdx.x == 0) sc[1] = a.first ? 0.0 : sc[0] / rl(*a.rho0);
   __syncthreads();
   const double rho = sc[0];
   if (a.first) {
@@ -1116,10 +1165,7 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
   }
   if (!barrier()) return;
   // 5: q -= BU (U^H q), p^H q
-  if (wid <= (GEP ? 1 : 0)) {
-    const T t = md_sum_partials(pc + (long)wid * g, g, lane);
-    if (lane == 0) ys[wid] = t;
-  }
+  total((const T*)pc, vc == 0 ? (GEP ? 2 : 1) : 0, ys);
   __syncthreads();
   const T uq = ys[0];
   {
@@ -1134,13 +1180,8 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
   }
   if (!barrier()) return;
   // 6: r -= (rho / p^H q) q, r^H r
-  if (wid == 0) {
-    const double t = md_sum_partials((const double*)pd, g, lane);
-    if (lane == 0) {
-      sc[0] = t;
-      sc[1] = -1.0 * (rho / t);
-    }
-  }
+  total((const double*)pd, vc == 0 ? 1 : 0, sc);
+  if (threadIdx.x == 0) sc[1] = -1.0 * (rho / sc[0]);
   __syncthreads();
   const double al = sc[1];
   double dot[1] = {0.0};
