@@ -314,9 +314,10 @@ JDG_API int jdgpu_dpjd_batch(int nprob, const int* n, double* const* a, int* con
  * blocks must save to be used, default 1e-4), "drop_schur" (drop tolerance of the Schur-complement fill; negative:
  * DROPTOL/10), "apply_graph" (1: jdgpu_dildl_apply replays the captured CUDA
  * graph of the application, as the eigensolver does), "fuse_inner" (1,
- * default: with the built-in matvec the inner CG/sQMR iteration keeps its
- * scalars on the device and synchronises once per iteration, same arithmetic;
- * 0: one synchronisation per scalar), "revcom_device" (1: reverse-
+ * default: with the built-in matvec the inner CG/sQMR iteration synchronises
+ * once, in one kernel where the size allows it, same arithmetic; 0: the matvec
+ * as a call of its own and two synchronisations, as with a caller's matvec),
+ * "revcom_device" (1: reverse-
  * communication requests on device pointers, see jdgpu_revcom_device_ptr),
  * "matching" (1: the first level of the factor takes its pivot and dropping
  * decisions in the symmetric scale of a maximum-product matching, the role of

@@ -214,33 +214,21 @@ def _revcom(complex_, kind, A, neig, matvec, precond=None, sigma=0.0, isearch=0,
     gep = B is not None or bmatvec is not None
     if kind == "pjd" and gep:
         b, jb, ib = _matrix(B, dt)
+    # the driver and its arguments (the same arrays in every call of the loop)
+    tail = [_p(s.IPRINT), _p(s.INFO), _p(s.GAP)]
+    solve = [_p(s.EIGS), _p(s.RES), _p(X), _p(s.lx), _p(s.NEIG), _p(s.SIGMA), _p(s.ISEARCH), _p(s.NINIT),
+             _p(s.MADSPACE), _p(s.ITER), _p(s.TOL)]
+    job = [_p(s.IJOB), _p(s.NDX[0:1]), _p(s.NDX[1:2])] + ([_p(s.NDX[2:3])] if gep else [])
+    if kind == "pjd":
+        mats = [_p(s.n), _p(a), _p(ja), _p(ia)] + ([_p(b), _p(jb), _p(ib)] if gep else [])
+        args = mats + solve + [_p(s.SHIFT), _p(s.DROPTOL), _p(s.MEM), _p(s.ICNTL)] + job + tail
+    else:
+        args = [_p(s.n)] + solve + job + tail
+    driver = getattr(L, pre + kind + "revcom" + ("_gep_" if gep else "_"))
     while True:
         if first and device:  # the mode is taken when the solve starts (IJOB = 0)
             L.jdgpu_set_option(b"revcom_device", C.c_double(1.0))
-        if kind == "pjd":
-            if gep:
-                getattr(L, pre + "pjdrevcom_gep_")(
-                    _p(s.n), _p(a), _p(ja), _p(ia), _p(b), _p(jb), _p(ib), _p(s.EIGS), _p(s.RES), _p(X), _p(s.lx),
-                    _p(s.NEIG), _p(s.SIGMA), _p(s.ISEARCH), _p(s.NINIT), _p(s.MADSPACE), _p(s.ITER), _p(s.TOL),
-                    _p(s.SHIFT), _p(s.DROPTOL), _p(s.MEM), _p(s.ICNTL), _p(s.IJOB), _p(s.NDX[0:1]), _p(s.NDX[1:2]),
-                    _p(s.NDX[2:3]), _p(s.IPRINT), _p(s.INFO), _p(s.GAP))
-            else:
-                getattr(L, pre + "pjdrevcom_")(
-                    _p(s.n), _p(a), _p(ja), _p(ia), _p(s.EIGS), _p(s.RES), _p(X), _p(s.lx), _p(s.NEIG), _p(s.SIGMA),
-                    _p(s.ISEARCH), _p(s.NINIT), _p(s.MADSPACE), _p(s.ITER), _p(s.TOL), _p(s.SHIFT), _p(s.DROPTOL),
-                    _p(s.MEM), _p(s.ICNTL), _p(s.IJOB), _p(s.NDX[0:1]), _p(s.NDX[1:2]), _p(s.IPRINT), _p(s.INFO),
-                    _p(s.GAP))
-        else:
-            if gep:
-                getattr(L, pre + "jdrevcom_gep_")(
-                    _p(s.n), _p(s.EIGS), _p(s.RES), _p(X), _p(s.lx), _p(s.NEIG), _p(s.SIGMA), _p(s.ISEARCH),
-                    _p(s.NINIT), _p(s.MADSPACE), _p(s.ITER), _p(s.TOL), _p(s.IJOB), _p(s.NDX[0:1]), _p(s.NDX[1:2]),
-                    _p(s.NDX[2:3]), _p(s.IPRINT), _p(s.INFO), _p(s.GAP))
-            else:
-                getattr(L, pre + "jdrevcom_")(
-                    _p(s.n), _p(s.EIGS), _p(s.RES), _p(X), _p(s.lx), _p(s.NEIG), _p(s.SIGMA), _p(s.ISEARCH),
-                    _p(s.NINIT), _p(s.MADSPACE), _p(s.ITER), _p(s.TOL), _p(s.IJOB), _p(s.NDX[0:1]), _p(s.NDX[1:2]),
-                    _p(s.IPRINT), _p(s.INFO), _p(s.GAP))
+        driver(*args)
         if first and device:
             L.jdgpu_set_option(b"revcom_device", C.c_double(0.0))
         first = False

@@ -400,106 +400,84 @@ correction:
       const bool one_launch = device_ops && k::inner_one_ok<T>(N, NEIG + 1, GEP);
       for (;;) {
         ++it;
-        if (device_ops) {
-          // The same operations in the same order in one kernel beside the
-          // preconditioner (k::inner_one, where the size allows it) or seven,
-          // with RHO, the projection coefficient, the B-inner product, P^H Q
-          // and |R|^2 read back together: one synchronisation per iteration.
-          // The checks on RHO and P^H Q come after the read; a failed check
-          // leaves Q, Z and R (and P after the first iteration) modified
-          // where the plain sequence stops earlier, and none of them is read
-          // after a failed inner solve.
-          precond(R, Zv);
-          S_.flagcg = true;
-          T* rho_d = scd + (it & 1);
-          const T* rho0_d = it > 1 ? scd + ((it - 1) & 1) : nullptr;
-          AXPYALPHA = H(-ETA);
-          H uq, buq;
-          double pq, rr;
-          const H* hs = reinterpret_cast<const H*>(W->hsm + kScal);
-          if (one_launch) {
-            const int parts = inner_one(NEIG + 1, UU, BU, Zv, R, P, -ETA, it == 1, POSDEF, rho_d, rho0_d);
-            sync();
-            if (hre(hs[4]) != (double)W->one.ticket) {
-              W->reset_barrier();
-              throw std::runtime_error("a grid barrier of the inner iteration ran out");
-            }
-            RHO = hre(hs[0]);
-            uq = hs[1];
-            buq = hs[2];
-            pq = hre(hs[3]);
-            rr = k::md_sum_host(W->hpart, parts);
-          } else {
-            k::mdot<T>(N, NEIG + 1, D(BU), N, D(Zv), W->dsm, W->dpart, S());
-            double* const be = reinterpret_cast<double*>(scd + 6);  // this iteration's two update scalars
-            double* const al = reinterpret_cast<double*>(scd + 7);
-            k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), rho_d, W->dpart, S(), nullptr, 0, nullptr, nullptr,
-                           rho0_d, rho0_d ? be : nullptr);
-            k::cg_direction<T>(N, rho_d, rho0_d ? be : nullptr, POSDEF, D(P), D(Zv), S());
-            matvec_shift(P, Q, Zv, -ETA);
-            k::mdot<T>(N, 1, D(UU), N, D(Q), scd + 2, W->dpart, S());
-            if (GEP) k::mdot<T>(N, 1, D(BU), N, D(Q), scd + 3, W->dpart, S());
-            k::gemv_dot<T>(N, 1, D(BU), N, scd + 2, D(Q), D(P), scd + 4, W->dpart, S(), nullptr, 0, nullptr, rho_d,
-                           nullptr, al);
-            k::cg_residual<T>(N, al, D(Q), D(R), scd + 5, scd, 6, W->hsm + kScal, W->dpart, S());
-            sync();
-            RHO = hre(hs[it & 1]);
-            uq = hs[2];
-            buq = hs[3];
-            pq = hre(hs[4]);
-            rr = hre(hs[5]);
-          }
-          if (POSDEF && RHO <= 0) {
-            std::fprintf(stderr, " Non fatal bug: the preconditioner is not positive definite\n");
-            fail = true;
-            break;
-          }
-          if (RHO == 0) { fail = true; break; }
-          if (GEP) AXPYALPHA = buq / (NBU * NBU);
-          X[NP] = uq;
-          ALPRHO = hre(X[NP]);
-          ITER++;
-          alpha_cg = pq;
-          if ((POSDEF && alpha_cg <= 0) || alpha_cg == 0) { fail = true; break; }
-          alpha_cg = RHO / alpha_cg;
-          GK = std::sqrt(rr);
-        } else {
+        // RHO, the projection coefficient, the B-inner product, P^H Q and |R|^2
+        // stay on the device and are read back together: one synchronisation
+        // per iteration with the built-in operators (in one kernel beside the
+        // preconditioner, k::inner_one, where the size allows it), one more
+        // before a caller's matvec, which is not asked for when RHO ends the
+        // solve.  A check that fails after the read leaves Q, Z and R (and P
+        // after the first iteration) modified where a sequence with a read
+        // per scalar stops earlier; none of them is read after a failed inner
+        // solve.
         precond(R, Zv);
         S_.flagcg = true;
-        if (NEIG + 1 > 64) throw std::runtime_error("projection against more than 64 vectors");
-        k::mdot<T>(N, NEIG + 1, D(BU), N, D(Zv), W->dsm, W->dpart, S());
-        k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), W->hsm + kScal, W->dpart, S());
-        sync();
-        RHO = hre(reinterpret_cast<const H*>(W->hsm + kScal)[0]);
+        T* rho_d = scd + (it & 1);
+        const T* rho0_d = it > 1 ? scd + ((it - 1) & 1) : nullptr;
+        AXPYALPHA = H(-ETA);
+        H uq, buq;
+        double pq, rr;
+        const H* hs = reinterpret_cast<const H*>(W->hsm + kScal);
+        if (one_launch) {
+          const int parts = inner_one(NEIG + 1, UU, BU, Zv, R, P, -ETA, it == 1, POSDEF, rho_d, rho0_d);
+          sync();
+          if (hre(hs[4]) != (double)W->one.ticket) {
+            W->reset_barrier();
+            throw std::runtime_error("a grid barrier of the inner iteration ran out");
+          }
+          RHO = hre(hs[0]);
+          uq = hs[1];
+          buq = hs[2];
+          pq = hre(hs[3]);
+          rr = k::md_sum_host(W->hpart, parts);
+        } else {
+          double* const be = reinterpret_cast<double*>(scd + 6);  // this iteration's two update scalars
+          double* const al = reinterpret_cast<double*>(scd + 7);
+          k::mdot<T>(N, NEIG + 1, D(BU), N, D(Zv), W->dsm, W->dpart, S());
+          k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), rho_d, W->dpart, S(), rho_d, device_ops ? 0 : 1,
+                         W->hsm + kScal, nullptr, rho0_d, rho0_d ? be : nullptr);
+          if (!device_ops) {
+            sync();
+            RHO = hre(hs[0]);
+            if ((POSDEF && RHO <= 0) || RHO == 0) {
+              if (RHO != 0 || POSDEF)
+                std::fprintf(stderr, " Non fatal bug: the preconditioner is not positive definite\n");
+              fail = true;
+              break;
+            }
+          }
+          k::cg_direction<T>(N, rho_d, rho0_d ? be : nullptr, POSDEF, D(P), D(Zv), S());
+          if (device_ops) {
+            matvec_shift(P, Q, Zv, -ETA);
+          } else {
+            matvec(1, P, Q, Zv);
+            axpy(N, AXPYALPHA, GEP ? Zv : P, Q);
+          }
+          k::mdot<T>(N, 1, D(UU), N, D(Q), scd + 2, W->dpart, S());
+          if (GEP) k::mdot<T>(N, 1, D(BU), N, D(Q), scd + 3, W->dpart, S());
+          k::gemv_dot<T>(N, 1, D(BU), N, scd + 2, D(Q), D(P), scd + 4, W->dpart, S(), nullptr, 0, nullptr, rho_d,
+                         nullptr, al);
+          k::cg_residual<T>(N, al, D(Q), D(R), scd + 5, scd, 6, W->hsm + kScal, W->dpart, S());
+          sync();
+          RHO = hre(hs[it & 1]);
+          uq = hs[2];
+          buq = hs[3];
+          pq = hre(hs[4]);
+          rr = hre(hs[5]);
+        }
         if (POSDEF && RHO <= 0) {
           std::fprintf(stderr, " Non fatal bug: the preconditioner is not positive definite\n");
           fail = true;
           break;
         }
         if (RHO == 0) { fail = true; break; }
-        if (it > 1) {
-          axpy(N, H(RHO / RHO1), P, Zv);
-          copy(N, Zv, P);
-        } else {
-          copy(N, Zv, P);
-        }
-        matvec(1, P, Q, Zv);
-        AXPYALPHA = H(-ETA);
-        if (GEP) axpy(N, AXPYALPHA, Zv, Q);
-        else axpy(N, AXPYALPHA, P, Q);
-        if (GEP) AXPYALPHA = dot(N, BU, Q) / (NBU * NBU);
-        k::mdot<T>(N, 1, D(UU), N, D(Q), W->dsm, W->dpart, S());
-        k::gemv_dot<T>(N, 1, D(BU), N, W->dsm, D(Q), D(P), W->dsm + 1, W->dpart, S(), W->dsm, 2, W->hsm + kScal);
-        sync();
-        X[NP] = reinterpret_cast<const H*>(W->hsm)[kScal];
+        if (GEP) AXPYALPHA = buq / (NBU * NBU);
+        X[NP] = uq;
         ALPRHO = hre(X[NP]);
         ITER++;
-        alpha_cg = hre(reinterpret_cast<const H*>(W->hsm)[kScal + 1]);
+        alpha_cg = pq;
         if ((POSDEF && alpha_cg <= 0) || alpha_cg == 0) { fail = true; break; }
         alpha_cg = RHO / alpha_cg;
-        axpy(N, H(-alpha_cg), Q, R);
-        GK = nrm2(N, R);
-        }
+        GK = std::sqrt(rr);
         if (!POSDEF) {
           double GK2 = GK * GK;
           TTK2M = TTK2;

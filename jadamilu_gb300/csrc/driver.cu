@@ -1331,15 +1331,36 @@ struct Revcom {
   bool cancel = false;
   bool device = false;  // requests served on the device copy of X
   std::string error;
+  // A hand-over takes two thread wake-ups (20 to 50 us each when the other
+  // side sleeps) around requests that are often shorter, so each side first
+  // watches a copy of the state for kSpin before it sleeps on the condition
+  // variable.  A solve with device
+  // requests, Anderson 24^3 (GB300): 45 -> 30 ms, with one read less per
+  // iteration and the Python loop's arguments made once.
+  std::atomic<int> seen{IDLE};
+  static constexpr std::chrono::microseconds kSpin{200};
+  template <class Pred> void watch(Pred pred) {
+    const auto until = std::chrono::steady_clock::now() + kSpin;
+    while (!pred(seen.load(std::memory_order_acquire)) && std::chrono::steady_clock::now() < until)
+      std::this_thread::yield();
+  }
+  void set(State s) {  // with m held
+    state = s;
+    seen.store(s, std::memory_order_release);
+    cv.notify_all();
+  }
   // worker side: post a request and wait for the caller to serve it
   void request(int job, long x1, long x2, long x3) {
+    {
+      std::lock_guard<std::mutex> lk(m);
+      ijob = job;
+      ndx1 = (int)x1 + 1;
+      ndx2 = (int)x2 + 1;
+      ndx3 = (int)x3 + 1;
+      set(REQUEST);
+    }
+    watch([](int s) { return s == RUNNING; });
     std::unique_lock<std::mutex> lk(m);
-    ijob = job;
-    ndx1 = (int)x1 + 1;
-    ndx2 = (int)x2 + 1;
-    ndx3 = (int)x3 + 1;
-    state = REQUEST;
-    cv.notify_all();
     cv.wait(lk, [&] { return state == RUNNING || cancel; });
     if (cancel) throw RevcomCancelled();
   }
@@ -1348,7 +1369,10 @@ struct Revcom {
     finish_old();
     cancel = false;
     error.clear();
-    state = RUNNING;
+    {
+      std::lock_guard<std::mutex> lk(m);
+      set(RUNNING);
+    }
     th = std::thread([this, body] {
       try {
         body();
@@ -1357,17 +1381,16 @@ struct Revcom {
         error = e.what();
       }
       std::lock_guard<std::mutex> lk(m);
-      state = DONE;
-      cv.notify_all();
+      set(DONE);
     });
   }
   void resume() {
     std::lock_guard<std::mutex> lk(m);
-    state = RUNNING;
-    cv.notify_all();
+    set(RUNNING);
   }
   // wait for the next request or the end; true when finished
   bool wait() {
+    watch([](int s) { return s == REQUEST || s == DONE; });
     std::unique_lock<std::mutex> lk(m);
     cv.wait(lk, [&] { return state == REQUEST || state == DONE; });
     if (state == DONE) {
