@@ -11,6 +11,7 @@
 #include <climits>
 #include <functional>
 #include <map>
+#include <type_traits>
 
 #include <mutex>
 
@@ -1572,7 +1573,17 @@ __global__ void __launch_bounds__(RUN_TPB) ildl_run_kernel(int l0, int l1, const
 }
 // One wide level: LANES lanes per row (8, 16 or 32, from the level's mean
 // row length, so long rows are read by more lanes at once).
-constexpr int WIDE_TPB = 256;
+//
+// Blocks of 128 threads free their SM slots in smaller pieces than 256 did, and
+// a float64 level lets its successor start only once it has its own y (LATE):
+// the successor's blocks, there to load their entries, otherwise take turns on
+// the FP64 units and slots this level still needs.  us per application (GB300),
+// 256 threads and early -> as here: FEM 384^2 float64 276 -> 238, tight-binding
+// 48^3 complex128 386 -> 277, complex64 139 -> 132, Anderson 44^3 float64 361 ->
+// 340, Laplacian 32^3 185 -> 181; early with 128 threads 268, 375, -, 357, 183;
+// float32 late: FEM 127.6 -> 131.5, Anderson 44^3 155.6 -> 156.8.
+constexpr int WIDE_TPB = 128;
+template <class A> constexpr bool kLate = sizeof(A) == 16 || std::is_same<A, double>::value;
 static inline int lanes_for(double entries_per_row) {
   return entries_per_row >= 48 ? 32 : entries_per_row >= 20 ? 16 : 8;
 }
@@ -1581,7 +1592,7 @@ template <class S, class A, int LANES>
 __global__ void __launch_bounds__(WIDE_TPB) ildl_wide_kernel(int lo, int hi, const int* __restrict__ rows,
                                                             const int64_t* __restrict__ rp, const int* __restrict__ ci,
                                                             const S* __restrict__ cv, A* __restrict__ y) {
-  pdl_launch();
+  if (!kLate<A>) pdl_launch();
   const int g = blockIdx.x * (WIDE_TPB / LANES) + (threadIdx.x / LANES);
   const int lane = threadIdx.x % LANES;
   const int t = lo + g;
@@ -1599,6 +1610,7 @@ __global__ void __launch_bounds__(WIDE_TPB) ildl_wide_kernel(int lo, int hi, con
   ent_load<false>(first, b, e, LANES, ci, cv);
   ent_load<false>(second, b + kUnr * LANES, e, LANES, ci, cv);
   pdl_wait();
+  if (kLate<A>) pdl_launch();
   const A own = ok && lane == 0 ? y[s] : A(0);  // requested with the gathers, not after the sum
   A acc = ent_pipe<false, kUnr>(first, b, e, LANES, ci, cv, second, (const A*)y, (longest + LANES - 1) / LANES);
   acc = row_sum<LANES>(acc, longest);
