@@ -270,9 +270,10 @@ main_loop:
   if (ritz_late) {
     T y[32];
     for (long c = 0; c < J; ++c) y[c] = todev(X[YY + c]);
+    mark(W->hsm, GEP ? 2 : 1);
     k::ritz<T>(N, (int)J, D(VV), D(WW), GEP ? D(BV) : nullptr, N, y, -THMT, D(UU), D(REIG),
                GEP ? D(BU) : nullptr, W->hsm, W->dpart, S());
-    sync();
+    await(W->hsm, GEP ? 2 : 1);
     NREIG = std::sqrt(rl(W->hsm[0]));
     if (GEP) NBU = std::sqrt(rl(W->hsm[1]));
   } else {
@@ -384,7 +385,10 @@ correction:
       S_.shift1 = THETA;
       GAP = (J > 1) ? THETA2 - THETA : 0;
     }
-    if (GEP) k::mdot<T>(N, 1, D(BU), N, D(REIG), W->hsm + kLate, W->dpart, S());
+    if (GEP) {
+      mark(W->hsm + kLate, 1);
+      k::mdot<T>(N, 1, D(BU), N, D(REIG), W->hsm + kLate, W->dpart, S());
+    }
     const long R = WCG, Zv = WCG + N, P = WCG + 2 * N, Q = WCG + 3 * N, X2 = XCG2, BTv = BT, Xc = XCG;
     bool FTFLG = true;
     {
@@ -417,9 +421,12 @@ correction:
         H uq, buq;
         double pq, rr;
         const H* hs = reinterpret_cast<const H*>(W->hsm + kScal);
+        mark(W->hsm + kScal, 6);
         if (one_launch) {
+          mark(W->hpart, k::reduction_blocks(N));
           const int parts = inner_one(NEIG + 1, UU, BU, Zv, R, P, -ETA, it == 1, POSDEF, rho_d, rho0_d);
-          sync();
+          await(W->hsm + kScal, 5);
+          await(W->hpart, parts);
           if (hre(hs[4]) != (double)W->one.ticket) {
             W->reset_barrier();
             throw std::runtime_error("a grid barrier of the inner iteration ran out");
@@ -436,7 +443,7 @@ correction:
           k::gemv_dot<T>(N, NEIG + 1, D(UU), N, W->dsm, D(Zv), D(R), rho_d, W->dpart, S(), rho_d, device_ops ? 0 : 1,
                          W->hsm + kScal, nullptr, rho0_d, rho0_d ? be : nullptr);
           if (!device_ops) {
-            sync();
+            await(W->hsm + kScal, 1);
             RHO = hre(hs[0]);
             if ((POSDEF && RHO <= 0) || RHO == 0) {
               if (RHO != 0 || POSDEF)
@@ -456,8 +463,9 @@ correction:
           if (GEP) k::mdot<T>(N, 1, D(BU), N, D(Q), scd + 3, W->dpart, S());
           k::gemv_dot<T>(N, 1, D(BU), N, scd + 2, D(Q), D(P), scd + 4, W->dpart, S(), nullptr, 0, nullptr, rho_d,
                          nullptr, al);
+          if (!device_ops) mark(W->hsm + kScal, 6);
           k::cg_residual<T>(N, al, D(Q), D(R), scd + 5, scd, 6, W->hsm + kScal, W->dpart, S());
-          sync();
+          await(W->hsm + kScal, 6);
           RHO = hre(hs[it & 1]);
           uq = hs[2];
           buq = hs[3];
@@ -489,7 +497,10 @@ correction:
                          it == 1 ? alpha_cg * CK2 : TTK2M * CK2, D(P), D(X2), D(Xc), alpha_cg, D(Zv),
                          GEP ? D(BTv) : nullptr, S());
         if (FTFLG) IFO = (ISERCH == 2) ? -2 : -1;
-        if (FTFLG && GEP) AXPYBETA = reinterpret_cast<const H*>(W->hsm)[kLate] / (NBU * NBU);
+        if (FTFLG && GEP) {
+          await(W->hsm + kLate, 1);
+          AXPYBETA = reinterpret_cast<const H*>(W->hsm)[kLate] / (NBU * NBU);
+        }
         AXPYALPHA *= alpha_cg;
         ALPRHO *= alpha_cg;
         stoptest(N, Xc, BTv, BU, TOL, RESID, NBU, ALPRHO, GK, AXPYALPHA, AXPYBETA, THETA, ETA, IFO, TRS, GEP);
@@ -504,7 +515,7 @@ correction:
         if (it == 1) copy(N, P, Xc);
       }
     }
-    RNDIND = habs(repgs_coef(NEIG)) / (NREIG * EPSMSR);  // every inner iteration has synchronised
+    RNDIND = habs(repgs_coef(NEIG)) / (NREIG * EPSMSR);
     if (ISERCH != 2 && ETA <= ETA0 && NEIG > 0 && IFO == 2) ETA0 = std::min(ETA1, ETA0);
     CONV = false;
     S_.flagcg = false;

@@ -378,6 +378,8 @@ static inline int md_grid(long n) {
   return (int)std::min<long>((n + 511) / 512, kMaxPartials);
 }
 
+int reduction_blocks(long n) { return md_grid(n); }
+
 // The partials follow one arrival counter per column group at the start of
 // the buffer (zero when the buffer is allocated; the last CTA of a group
 // resets its counter).

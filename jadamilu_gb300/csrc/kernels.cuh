@@ -136,6 +136,7 @@ template <class T> void fill(long n, T v, T* x, cudaStream_t s);
 // mdot_partial_size(n,k) entries
 constexpr int kPartialHead = 16;  // entries before the partials: the arrival counters
 long mdot_partial_size(long n, int k);
+int reduction_blocks(long n);  // CTAs of a reduction over n rows
 template <class T>
 void mdot(long n, int k, const T* V, long ldv, const T* w, T* out, T* partial, cudaStream_t s, const T* xcol = nullptr);
 // w = beta*w + alpha*V*y (alpha and beta real), y (k <= 64 entries) in device memory (copied to the
