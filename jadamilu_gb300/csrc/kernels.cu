@@ -4,8 +4,9 @@
 // path): SpMV over the full Hermitian matrix in SELL-32 layout (coalesced
 // column/value loads), the level-scheduled sweeps of the multilevel LDL^H
 // preconditioner, and the BLAS-1/2 vector work of the outer and inner JD
-// iterations (deterministic two-pass reductions, so results do not depend on
-// the launch).
+// iterations (deterministic reductions, so results do not depend on timing).
+// Short problems are bound by launches and dependent latencies instead, float64
+// ones also by the FP64 units; each kernel says which.
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -355,8 +356,6 @@ __device__ __forceinline__ float shfl_xor_any(float v, int o) { return __shfl_xo
 __device__ __forceinline__ double shfl_xor_any(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ cc shfl_xor_any(cc v, int o) { return cc(shfl_xor_any(v.x, o), shfl_xor_any(v.y, o)); }
 __device__ __forceinline__ zc shfl_xor_any(zc v, int o) { return zc(shfl_xor_any(v.x, o), shfl_xor_any(v.y, o)); }
-__device__ __forceinline__ double shfl_idx_any(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
-__device__ __forceinline__ zc shfl_idx_any(zc v, int l) { return zc(shfl_idx_any(v.x, l), shfl_idx_any(v.y, l)); }
 
 // loads that bypass L1 (data another CTA of the same launch wrote)
 __device__ __forceinline__ double ldcg_(const double* p) { return __ldcg(p); }
@@ -907,15 +906,14 @@ int* wait_expired_flag() {
 }
 
 // ------------------------------------ the inner iteration in one launch ----
-// The kernels above as the phases of one kernel.  Up to 1e5
-// rows a phase's bytes take well under a microsecond, and each kernel
-// pays a launch and, most of them, a reduction tail (fence, atomic, partials
-// read back: 3 us).  Here a phase ends in one barrier of the grid; its partial
-// sums go to a buffer and every CTA adds them up itself in the
-// order of md_finish, so there is no tail; the last reduction's partials go to
-// pinned memory and are added by the host the same way.  A physical CTA holds
-// VC of mdot's CTAs (256 threads each), so the order of every sum is that of
-// the separate kernels.
+// The kernels above as the phases of one kernel.  Up to 1e5 rows a phase's bytes
+// take well under a microsecond, and each kernel pays a launch and, most of
+// them, a reduction tail (fence, atomic, partials read back: 3 us).  Here a
+// phase ends in one barrier of the grid; its partial sums go to a buffer and
+// every CTA adds them up itself in the order of md_finish, so there is no tail;
+// the last reduction's partials go to pinned memory and are added by the host
+// the same way.  A physical CTA holds VC of mdot's CTAs (256 threads each), so
+// the order of every sum is that of the separate kernels.
 // Bound: the chain of six phases, each a barrier, a few L2 latencies (0.14 us)
 // and dependent float64 additions (some 50 cycles each), and from 1e5 rows on
 // the FP64 units (2 FMA per SM and cycle).  us per iteration with 5 columns,
@@ -923,7 +921,6 @@ int* wait_expired_flag() {
 // 64000 46.8 -> 26.7, 262144 59.3 -> 50.3, complex 262144 109 -> 102.
 constexpr int kOneMaxCols = GMV_MAX;
 constexpr int kBarPolls = 1 << 22;
-int inner_one_partials(long n, int k) { return md_grid(n) * (k + 3); }
 
 // Grid barrier of a cooperative launch: the counter only grows, by gridDim.x
 // per barrier, and `target` is its value once every CTA has arrived.  Gives up
@@ -957,7 +954,7 @@ template <class T> struct InnerOne {
   bool first, posdef;
   T *rho, *hsc;
   const T* rho0;                // the previous iteration's rho (not read in the first)
-  T* part;                      // inner_one_partials(n, k) entries
+  T* part;                      // (k + 3) g entries
   double* hpart;                // pinned, g entries: the partials of r^H r
   unsigned* bar;
   unsigned base;                // the barrier counter before this launch
@@ -1577,13 +1574,18 @@ __global__ void __launch_bounds__(RUN_TPB) ildl_run_kernel(int l0, int l1, const
 // row length, so long rows are read by more lanes at once).
 //
 // Blocks of 128 threads free their SM slots in smaller pieces than 256 did, and
-// a float64 level lets its successor start only once it has its own y (LATE):
+// a float64 level lets its successor start only once it has its own y (kLate):
 // the successor's blocks, there to load their entries, otherwise take turns on
 // the FP64 units and slots this level still needs.  us per application (GB300),
 // 256 threads and early -> as here: FEM 384^2 float64 276 -> 238, tight-binding
 // 48^3 complex128 386 -> 277, complex64 139 -> 132, Anderson 44^3 float64 361 ->
 // 340, Laplacian 32^3 185 -> 181; early with 128 threads 268, 375, -, 357, 183;
-// float32 late: FEM 127.6 -> 131.5, Anderson 44^3 155.6 -> 156.8.
+// float32 late: FEM 127.6 -> 131.5, Anderson 44^3 155.6 -> 156.8.  A float64 tile
+// product (tri_cluster_kernel) lets it start once its products are done: FEM
+// 384^2 239 -> 232, Anderson 36^3 269 -> 261.5, a FEM 512^2 solve 214.5 -> 211.1
+// ms, Laplacian 20^3 30.2 -> 29.7.  A level that waits for its products, too, is
+// faster when applications follow one another (FEM 384^2 238 -> 234) but not in a
+// solve (FEM 512^2 226.9 ms): its successor then asks for its entries too late.
 constexpr int WIDE_TPB = 128;
 template <class A> constexpr bool kLate = sizeof(A) == 16 || std::is_same<A, double>::value;
 static inline int lanes_for(double entries_per_row) {
@@ -1819,7 +1821,7 @@ template <class S, class A, int CL>
 __global__ void __launch_bounds__(TRI_TPB)
     tri_cluster_kernel(const int4* __restrict__ items, bool rev, const S* __restrict__ tiles, const A* __restrict__ x,
                        int m, A* __restrict__ y) {
-  pdl_launch();
+  if (!kLate<A>) pdl_launch();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   constexpr int V = 16 / sizeof(S);
@@ -1888,6 +1890,7 @@ __global__ void __launch_bounds__(TRI_TPB)
 #pragma unroll
     for (int j = 1; j < CPS; ++j) sum = sum + red[j][threadIdx.x];
   }
+  if (kLate<A>) pdl_launch();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (threadIdx.x < 64) *cl.map_shared_rank(&part[cl.block_rank()][threadIdx.x], 0) = sum;
   cl.sync();

@@ -169,13 +169,12 @@ void cg_residual(long n, const double* al, const T* q, T* r, T* out, const T* sc
 // allow it: r and p as there, z = B p with B (else left alone), rho (device, this iteration's), and on the host after
 // the stream has synchronised hsc[0..4] = rho, U^H q, BU^H q (with B), p^H q, st.ticket (as the call left it; anything
 // else: a barrier gave up) and hpart[0..g) the partials of r^H r, g the return value, to be added by md_sum_host.
-// part: inner_one_partials(n, k) entries; bar: a counter that starts at zero, with st.base = 0, and is only used here.
+// part: (k + 3) * reduction_blocks(n) entries; bar: a counter that starts at zero, with st.base = 0, and is only used here.
 struct OneState {
   unsigned base = 0;    // what the barrier counter holds
   unsigned ticket = 0;  // launches so far
 };
 template <class T> bool inner_one_ok(long n, int k, bool gep);
-int inner_one_partials(long n, int k);
 constexpr int kMaxPartials = 152 * 8;  // most CTAs of a reduction
 double md_sum_host(const double* p, int g);
 template <class T>
