@@ -133,7 +133,9 @@ void build_sell_host(int n, const int* ia, const int* ja, const H* a, SellMatrix
   CK(cudaStreamSynchronize(st));
 }
 // The matrix for the products from the caller's triangle; keep: a staging
-// buffer that outlives the call (a solver's), else one of its own.
+// buffer that outlives the call (a solver's), else one of its own.  Returns
+// with the matrix complete: the products load it before they wait for their
+// predecessor, so its writers must not be in flight when one is launched.
 template <class T, class H>
 void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, cudaStream_t st,
                 SellStage* keep = nullptr) {
@@ -158,7 +160,7 @@ void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& 
   if (built) {
     M.stored = (int64_t)info[0];
     M.nnz = (int64_t)info[1];
-    if (!keep) CK(cudaStreamSynchronize(st));  // the staging buffer goes
+    CK(cudaStreamSynchronize(st));
   } else {
     build_sell_host<T>(n, ia, ja, a, M, st);
   }

@@ -39,9 +39,14 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// The two halves of pdl_begin, for kernels that load their factor data
-// (never written while the preconditioner runs) before waiting for the
-// predecessor's results: those loads overlap the predecessor's tail.
+// The two halves of pdl_begin, for kernels that load data before waiting for
+// the predecessor's results: those loads overlap the predecessor's tail.  They
+// are ordered after no kernel of the stream but those complete at its last full
+// ordering point (a synchronisation, a copy, a launch without the attribute): a
+// predecessor that released its successor at its start may itself still wait for
+// the kernel before it.  So they may touch only data that is finished before
+// the kernels that read it are launched: the factor (upload_factor ends in a
+// synchronisation), the matrix (build_sell does) and its slice pointers.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Asks the TMA unit to bring [p, p + bytes) into L2 and returns at once (a
@@ -301,6 +306,7 @@ bool sell_from_triangle(int n, const int* ia, const int* ja, const void* a, void
   int* col = nullptr;
   T* val = nullptr;
   room((int64_t)info_host[0], &col, &val);
+  // the caller synchronises before a product reads what these write (see pdl_launch)
   launch_k(sell_fill_kernel<T>, g, t, 0, s, n, dia, dja, sptr, cur, val);
   launch_k(sell_finish_kernel<T>, g, t, 0, s, n, dia, dja, da, sptr, tcnt, col, val);
   g_launches += 5;

@@ -119,7 +119,7 @@ int* wait_expired_flag();
 // layout).  work: sell_work_bytes(n, nnz, sizeof(T)) device bytes; sptr: (n + 31) / 32 + 1 entries; info_host: 4
 // entries, then stored slots and full nonzeros in the first two; room: called once, after a synchronisation, with the
 // slots needed, gives the col and val arrays.  False (nothing built): a row too long for it, use the host pass.  The
-// host arrays are read before it returns.
+// host arrays are read before it returns; the last kernels are then still in flight: synchronise before a product.
 int64_t sell_work_bytes(int n, int64_t nnz, int64_t value);
 template <class T>
 bool sell_from_triangle(int n, const int* ia, const int* ja, const void* a, void* work, int64_t* sptr,
