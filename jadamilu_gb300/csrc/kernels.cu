@@ -1407,8 +1407,11 @@ __device__ __forceinline__ A ent_use(const EntBatch<A, U>& b, const A* y, A acc,
 // the SM's FP64 unit for 16 cycles per warp whether its lanes are zero or not.
 // us per application (GB300): tridiagonal n = 1000 28.7 -> 22.6, FEM 384^2 291
 // -> 276, Anderson 56^3 350 -> 339, 40^3 151 -> 149, Laplacian 20^3 58.2 -> 56.7.
+// Lengths are exact up to kLongest, which no caller reaches: batch counts
+// derived from a smaller cap would drop the entries beyond it.
+constexpr int kLongest = 1 << 30;
 __device__ __forceinline__ int warp_longest(int64_t len) {
-  return __reduce_max_sync(0xffffffffu, (int)(len < 0 ? 0 : len < 4096 ? len : 4096));
+  return __reduce_max_sync(0xffffffffu, (int)(len < 0 ? 0 : len < kLongest ? len : kLongest));
 }
 template <int LANES, class A> __device__ __forceinline__ A row_sum(A v, int longest) {
 #pragma unroll
