@@ -147,6 +147,9 @@ void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& 
   } own;
   SellStage& stage = keep ? *keep : own;
   const int ns = (n + 31) / 32;
+  // no matrix until its arrays are complete: a refused one leaves foreign slice pointers behind
+  M.n = M.nslices = 0;
+  M.nnz = M.stored = 0;
   sell_slices(M, ns);
   unsigned long long info[4] = {};
   const bool built = k::sell_from_triangle<T>(
@@ -1999,6 +2002,7 @@ JDG_API int jdgpu_dprepare_matrix(int n, const int* ia, const int* ja, const dou
   try {
     Global<double>& g = G<double>();
     g.W.ensure(n, n);
+    g.resident = false;  // until the new one is there: the build overwrites the one prepared before
     build_sell<double>(n, ia, ja, a, g.A, g.W.st, &g.stage);
     g.resident = true;
     return 0;

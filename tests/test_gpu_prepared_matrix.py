@@ -1,0 +1,43 @@
+"""A matrix prepared on the device for several solves: what becomes of it when
+a later one is refused."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from jadamilu_gb300 import matrices as M
+
+pytestmark = pytest.mark.gpu
+
+KW = dict(isearch=0, madspace=20, maxit=2000, tol=1e-10, droptol=1e-3, icntl=(0, 1, 0, 0, 0))
+
+
+def _rows_held(gpu):
+    out = np.zeros(3, np.int64)
+    gpu.load().jdgpu_dmatrix_info(out.ctypes.data_as(C.c_void_p))
+    return int(out[2])
+
+
+@pytest.mark.parametrize("bad", [0, 1 << 30])
+def test_refused_matrix_is_not_used(gpu, bad):
+    """A refused matrix (a column out of range) of another row structure must
+    not leave its slice pointers to solves with the one prepared before."""
+    ia, ja, a = M.laplace3d(12)
+    plain = gpu.dpjd((a.copy(), ja.copy(), ia), 3, **KW)
+    assert plain["info"] == 0
+    n = len(ia) - 1
+    ib = np.arange(1, 40 * n + 2, 40, dtype=np.int32)  # 40 entries per row
+    jb = (np.arange(40 * n) % n + 1).astype(np.int32)
+    jb[-1] = bad
+    try:
+        gpu.prepare_matrix((a, ja, ia))
+        assert _rows_held(gpu) == n
+        with pytest.raises(RuntimeError):
+            gpu.prepare_matrix((np.ones(40 * n), jb, ib))
+        assert _rows_held(gpu) == 0
+        r = gpu.dpjd((a.copy(), ja.copy(), ia), 3, **KW)
+    finally:
+        gpu.release_matrix()
+    assert r["info"] == 0 and r["x"].shape == (n, 3)
+    np.testing.assert_array_equal(r["eigs"], plain["eigs"])
+    np.testing.assert_array_equal(r["x"], plain["x"])
