@@ -55,8 +55,12 @@ template <class T> struct Workspace {
     one.base = 0;
   }
   bool own_stream = false;
+  // Every entry leaves its stream idle (Idle), so a caller's stream needs no wait here
   void set_stream(cudaStream_t s) {
-    if (own_stream && st) cudaStreamDestroy(st);
+    if (own_stream && st) {
+      cudaStreamSynchronize(st);
+      cudaStreamDestroy(st);
+    }
     st = s;
     own_stream = false;
   }
@@ -111,6 +115,16 @@ template <class T> struct Workspace {
     cap_x = cap_tmp = cap_part = 0;
   }
   ~Workspace() {}
+};
+
+// Waits for the workspace's stream at the end of a scope, exceptions included: a
+// kernel still in flight could write host words that the next solve watches,
+// or work on buffers that it hands to another stream.
+template <class T> struct Idle {
+  Workspace<T>& W;
+  ~Idle() {
+    if (W.st) cudaStreamSynchronize(W.st);
+  }
 };
 
 template <class T> struct StopStateD {

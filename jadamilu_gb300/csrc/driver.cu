@@ -1172,6 +1172,7 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
     else std::printf("Computing the eigenvalue(s) closest to %12.5E\n---------------------------------------------------\n", SIGMA);
   }
   long lxl = LX;
+  Idle<T> idle{g.W};
   g.W.ensure(n, lxl);
   int ierr = 0;
   if ((ICNTL[1] != -1 && ICNTL[1] != -2) || g.factdgl == 0) {
@@ -1307,6 +1308,7 @@ void jd_drive(int n, double* EIGS, double* RES, typename HostOf<T>::type* X, int
               int ISEARCH, int NINIT, int MADSPACE, int* ITER, double TOL, int IPRINT, int* INFO, double* GAP,
               bool gep, std::function<void(int, long, long, long)> user_mv, std::function<void(long, long)> user_pc) {
   Global<T>& g = G<T>();
+  Idle<T> idle{g.W};
   g.W.ensure(n, LX);
   if (NINIT > 0)
     CK(cudaMemcpyAsync(g.W.dX, X, sizeof(T) * (size_t)n * NINIT, cudaMemcpyHostToDevice, g.W.st));
@@ -2001,6 +2003,7 @@ JDG_API int jdgpu_dildl_bench(int n, const int* ia, const int* ja, const double*
 JDG_API int jdgpu_dprepare_matrix(int n, const int* ia, const int* ja, const double* a) {
   try {
     Global<double>& g = G<double>();
+    Idle<double> idle{g.W};
     g.W.ensure(n, n);
     g.resident = false;  // until the new one is there: the build overwrites the one prepared before
     build_sell<double>(n, ia, ja, a, g.A, g.W.st, &g.stage);

@@ -41,3 +41,30 @@ def test_refused_matrix_is_not_used(gpu, bad):
     assert r["info"] == 0 and r["x"].shape == (n, 3)
     np.testing.assert_array_equal(r["eigs"], plain["eigs"])
     np.testing.assert_array_equal(r["x"], plain["x"])
+
+
+def test_stream_replaced_between_prepare_and_solve(gpu):
+    """The stream changes after the hand-over, after a solve and after one that
+    ends by an error (more basis vectors than a restart takes), each time with
+    work just done on the stream that goes; a kept factor leaves little host work
+    in between."""
+    torch = pytest.importorskip("torch")
+    ia, ja, a = M.laplace3d(24)
+    kept = dict(KW, icntl=(0, -1, 0, 0, 0))
+    plain = gpu.dpjd((a.copy(), ja.copy(), ia), 3, **KW)
+    assert plain["info"] == 0
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    try:
+        for k in range(6):
+            gpu.release_matrix()
+            r = gpu.dpjd((a.copy(), ja.copy(), ia), 3, **dict(kept, madspace=40))
+            assert r["info"] == -54330
+            gpu.set_stream(streams[k % 2].cuda_stream)
+            gpu.prepare_matrix((a, ja, ia))
+            gpu.set_stream(streams[(k + 1) % 2].cuda_stream if k % 3 else 0)
+            r = gpu.dpjd((a.copy(), ja.copy(), ia), 3, **kept)
+            assert r["info"] == 0
+            np.testing.assert_array_equal(r["eigs"], plain["eigs"])
+    finally:
+        gpu.set_stream(0)
+        gpu.release_matrix()
