@@ -35,6 +35,11 @@ static double wall() {
 }
 
 // --------------------------------------------------------- device matrix ----
+// Runs at the end of a scope, exceptions included.
+struct AtExit {
+  std::function<void()> f;
+  ~AtExit() { f(); }
+};
 // device buffer for the caller's triangle while a matrix is built from it
 struct SellStage {
   void* p = nullptr;
@@ -1810,21 +1815,28 @@ JDG_API int jdgpu_device_count(void) {
 }
 
 // y = A x with A given like DPJD's (upper, 1-based); x, y host arrays.
-JDG_API int jdgpu_dspmv(int n, const int* ia, const int* ja, const double* a, const double* x, double* y) {
-  try {
-    cudaStream_t st = nullptr;
-    SellMatrix<double> M;
-    build_sell<double>(n, ia, ja, a, M, st);
-    double *dx, *dy;
-    CK(cudaMalloc(&dx, sizeof(double) * n));
-    CK(cudaMalloc(&dy, sizeof(double) * n));
-    CK(cudaMemcpy(dx, x, sizeof(double) * n, cudaMemcpyHostToDevice));
-    k::spmv<double>(M, dx, dy, st);
-    CK(cudaGetLastError());
-    CK(cudaMemcpy(y, dy, sizeof(double) * n, cudaMemcpyDeviceToHost));
+extern "C++" {
+template <class T, class H> static void spmv_host(int n, const int* ia, const int* ja, const H* a, const H* x, H* y) {
+  cudaStream_t st = nullptr;
+  SellMatrix<T> M;
+  T *dx = nullptr, *dy = nullptr;
+  AtExit gone{[&] {
     cudaFree(dx);
     cudaFree(dy);
     free_sell(M);
+  }};
+  build_sell<T>(n, ia, ja, a, M, st);
+  CK(cudaMalloc(&dx, sizeof(T) * n));
+  CK(cudaMalloc(&dy, sizeof(T) * n));
+  CK(cudaMemcpy(dx, x, sizeof(T) * n, cudaMemcpyHostToDevice));
+  k::spmv<T>(M, dx, dy, st);
+  CK(cudaGetLastError());
+  CK(cudaMemcpy(y, dy, sizeof(T) * n, cudaMemcpyDeviceToHost));
+}
+}  // extern "C++"
+JDG_API int jdgpu_dspmv(int n, const int* ia, const int* ja, const double* a, const double* x, double* y) {
+  try {
+    spmv_host<double>(n, ia, ja, a, x, y);
     return 0;
   } catch (std::exception& e) {
     std::fprintf(stderr, "jdgpu_dspmv: %s\n", e.what());
@@ -1833,19 +1845,7 @@ JDG_API int jdgpu_dspmv(int n, const int* ia, const int* ja, const double* a, co
 }
 JDG_API int jdgpu_zspmv(int n, const int* ia, const int* ja, const zh* a, const zh* x, zh* y) {
   try {
-    cudaStream_t st = nullptr;
-    SellMatrix<zc> M;
-    build_sell<zc>(n, ia, ja, a, M, st);
-    zc *dx, *dy;
-    CK(cudaMalloc(&dx, sizeof(zc) * n));
-    CK(cudaMalloc(&dy, sizeof(zc) * n));
-    CK(cudaMemcpy(dx, x, sizeof(zc) * n, cudaMemcpyHostToDevice));
-    k::spmv<zc>(M, dx, dy, st);
-    CK(cudaGetLastError());
-    CK(cudaMemcpy(y, dy, sizeof(zc) * n, cudaMemcpyDeviceToHost));
-    cudaFree(dx);
-    cudaFree(dy);
-    free_sell(M);
+    spmv_host<zc>(n, ia, ja, a, x, y);
     return 0;
   } catch (std::exception& e) {
     std::fprintf(stderr, "jdgpu_zspmv: %s\n", e.what());
@@ -2333,9 +2333,20 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
                                int maxit, double* grad, double* out) {
   if (n <= 1 || !ia || !ja || !a || !xin || !g || !grad || maxit < 1) return -1;
   try {
-    cudaStream_t st;
-    CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    cudaStream_t st = nullptr;
     SellMatrix<double> Am;
+    DevFactor<double> D;
+    unsigned char* base = nullptr;
+    double* hsm = nullptr;
+    AtExit gone{[&] {
+      if (st) cudaStreamSynchronize(st);
+      cudaFree(base);
+      if (hsm) cudaFreeHost(hsm);
+      free_factor(D);
+      free_sell(Am);
+      if (st) cudaStreamDestroy(st);
+    }};
+    CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     build_sell<double>(n, ia, ja, a, Am, st);
     IldlcParams p;
     p.droptol = droptol;
@@ -2352,24 +2363,17 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
     } else {
       ierr = ildlc_factor<double>(n, ia, ja, a, lambda, nullptr, nullptr, nullptr, p, F);
     }
-    if (ierr) {
-      free_sell(Am);
-      cudaStreamDestroy(st);
-      return ierr;
-    }
-    DevFactor<double> D;
+    if (ierr) return ierr;
     upload_factor(F, D, st);
     const size_t vb = sizeof(double) * n;
     enum { X, BX, G, R1, R2, Y, V, W, W1, W2, MU, T1, T2, BD, NV };
     // one allocation: the vectors, the scalars and the reduction's partials
     const size_t vs = (vb + 255) / 256 * 256, ps = sizeof(double) * k::mdot_partial_size(n, 1);
-    unsigned char* base = nullptr;
     CK(cudaMalloc(&base, vs * NV + 256 + ps));
     std::vector<double*> vec(NV);
     for (int k = 0; k < NV; ++k) vec[k] = (double*)(base + vs * k);
     double* const dsm = (double*)(base + vs * NV);
     double* const dpart = (double*)(base + vs * NV + 256);
-    double* hsm = nullptr;
     CK(cudaMallocHost(&hsm, sizeof(double) * 8));
     CK(cudaMemsetAsync(dpart, 0, ps, st));
     CK(cudaMemcpyAsync(vec[X], xin, vb, cudaMemcpyHostToDevice, st));
@@ -2478,11 +2482,6 @@ JDG_API int jdgpu_deigvec_grad(int n, const int* ia, const int* ja, const double
       out[0] = it;
       out[1] = beta1 > 0 ? rnorm / beta1 : 0;
     }
-    cudaFree(base);
-    cudaFreeHost(hsm);
-    free_factor(D);
-    free_sell(Am);
-    cudaStreamDestroy(st);
     return 0;
   } catch (std::exception& e) {
     std::fprintf(stderr, "jdgpu_deigvec_grad: %s\n", e.what());
