@@ -317,6 +317,9 @@ JDG_API int jdgpu_dpjd_batch(int nprob, const int* n, double* const* a, int* con
  * default: with the built-in matvec the inner CG/sQMR iteration synchronises
  * once, in one kernel where the size allows it, same arithmetic; 0: the matvec
  * as a call of its own and two synchronisations, as with a caller's matvec),
+ * "barrier_polls" (default 2^22, seconds): polls of a thread block at a grid
+ * barrier of that kernel before it gives up; the solve then ends with INFO =
+ * -54330,
  * "revcom_device" (1: reverse-
  * communication requests on device pointers, see jdgpu_revcom_device_ptr),
  * "matching" (1: the first level of the factor takes its pivot and dropping

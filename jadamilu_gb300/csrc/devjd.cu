@@ -425,9 +425,8 @@ correction:
         if (one_launch) {
           mark(W->hpart, k::reduction_blocks(N));
           const int parts = inner_one(NEIG + 1, UU, BU, Zv, R, P, -ETA, it == 1, POSDEF, rho_d, rho0_d);
-          await(W->hsm + kScal, 5);
-          await(W->hpart, parts);
-          if (hre(hs[4]) != (double)W->one.ticket) {
+          // a CTA that gives up a barrier never writes its words of hpart
+          if (!await(W->hsm + kScal, 4) || !await(W->hpart, parts)) {
             W->reset_barrier();
             throw std::runtime_error("a grid barrier of the inner iteration ran out");
           }

@@ -177,22 +177,27 @@ template <class T> struct DevJd {
   // itself.  The host marks those words before the launch and watches them
   // instead of waiting for the stream: 2 us less per read (9 us from launch to
   // wake-up on GB300).  After kWatch (long kernels before it, an error, a value
-  // with the mark's bits) it waits for the stream after all.
+  // with the mark's bits) it waits for the stream after all; await returns
+  // whether all words were written then.
   static constexpr unsigned long long kMark = 0x7FF4DEADBEEF5A5AULL;  // a signalling NaN no kernel produces
   static constexpr std::chrono::microseconds kWatch{300};
   template <class V> static void mark(V* h, long n) {
     auto* w = reinterpret_cast<unsigned long long*>(h);
     for (long i = 0; i < n * (long)(sizeof(V) / 8); ++i) __atomic_store_n(w + i, kMark, __ATOMIC_RELEASE);
   }
-  template <class V> void await(const V* h, long n) {
+  template <class V> bool await(const V* h, long n) {
     const auto* w = reinterpret_cast<const unsigned long long*>(h);
+    const long words = n * (long)(sizeof(V) / 8);
     const auto until = std::chrono::steady_clock::now() + kWatch;
-    for (long i = 0; i < n * (long)(sizeof(V) / 8); ++i)
+    for (long i = 0; i < words; ++i)
       for (int t = 1; __atomic_load_n(w + i, __ATOMIC_ACQUIRE) == kMark; ++t)
         if (t % 256 == 0 && std::chrono::steady_clock::now() > until) {
           sync();
-          return;
+          for (; i < words; ++i)
+            if (__atomic_load_n(w + i, __ATOMIC_ACQUIRE) == kMark) return false;
+          return true;
         }
+    return true;
   }
 
   // ---- device primitives on X offsets ----

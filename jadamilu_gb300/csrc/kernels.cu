@@ -900,17 +900,6 @@ template <class T> void rmult(long n, int K, int keep, const T* V, long ldv, con
   COUNT_LAUNCH();
 }
 
-// Set when a bounded wait inside a kernel runs out (the kernel then returns
-// instead of hanging); read and cleared by the host at the end of a solve.
-// The address is looked up on every call: one kept in a static would go stale
-// when the context is torn down and the module loaded again.
-__device__ int g_wait_expired;
-int* wait_expired_flag() {
-  void* p = nullptr;
-  CK(cudaGetSymbolAddress(&p, g_wait_expired));
-  return (int*)p;
-}
-
 // ------------------------------------ the inner iteration in one launch ----
 // The kernels above as the phases of one kernel.  Up to 1e5 rows a phase's bytes
 // take well under a microsecond, and each kernel pays a launch and, most of
@@ -926,23 +915,21 @@ int* wait_expired_flag() {
 // separate kernels -> one (GB300): n = 4096 26.5 -> 20.5, 15625 29.8 -> 24.6,
 // 64000 46.8 -> 26.7, 262144 59.3 -> 50.3, complex 262144 109 -> 102.
 constexpr int kOneMaxCols = GMV_MAX;
-constexpr int kBarPolls = 1 << 22;
 
 // Grid barrier of a cooperative launch: the counter only grows, by gridDim.x
 // per barrier, and `target` is its value once every CTA has arrived.  Gives up
-// (false, in every thread) after kBarPolls polls.
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target) {
+// (false, in every thread) after `polls` polls.
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, int polls) {
   __shared__ bool ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
     bool there = false;
-    for (int t = 0; t < kBarPolls && !there; ++t) {
+    for (int t = 0; t < polls && !there; ++t) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
       there = (int)(v - target) >= 0;
     }
-    if (!there) g_wait_expired = 1;
     ok = there;
   }
   __syncthreads();
@@ -964,7 +951,7 @@ template <class T> struct InnerOne {
   double* hpart;                // pinned, g entries: the partials of r^H r
   unsigned* bar;
   unsigned base;                // the barrier counter before this launch
-  unsigned ticket;              // this launch's number, returned at its end
+  int polls;                    // after which a CTA gives up its wait, and leaves its partials unwritten
 };
 
 // x is written during the kernel: its loads stay out of the read-only path
@@ -1003,7 +990,7 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
       asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
       return true;
     }
-    return grid_barrier(a.bar, target += gridDim.x);
+    return grid_barrier(a.bar, target += gridDim.x, a.polls);
   };
   auto has = [&](int j) { return on && row0 + j * step < n; };
   // the sums of the first nc columns over this virtual CTA's threads, as md_finish
@@ -1205,7 +1192,6 @@ __global__ void __launch_bounds__(TPB * VC, 1) inner_one_kernel(const __grid_con
     a.hsc[1] = uq;
     a.hsc[2] = GEP ? ys[1] : T(0);
     a.hsc[3] = T(sc[0]);
-    a.hsc[4] = T((double)a.ticket);
   }
 }
 
@@ -1329,7 +1315,7 @@ int inner_one(const SellMatrix<T>& A, const SellMatrix<T>* B, int k, const T* U,
   a.hpart = hpart;
   a.bar = bar;
   a.base = st.base;
-  a.ticket = ++st.ticket;
+  a.polls = st.polls;
   const OneShape<T> o = one_shape<T>(one_pick<T>(A.n, B != nullptr), B != nullptr);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a.g + o.vc - 1) / o.vc);

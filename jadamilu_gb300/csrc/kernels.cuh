@@ -112,8 +112,6 @@ long long launch_count();
 // programmatic dependent launch between the preconditioner's kernels (default on)
 void set_pdl(bool on);
 void add_launches(long long n);
-// device flag that a kernel sets when a bounded wait inside it ran out
-int* wait_expired_flag();
 
 // SELL-32 of the full Hermitian matrix from the caller's host CSR of one triangle (1-based; a: n values of T's
 // layout).  work: sell_work_bytes(n, nnz, sizeof(T)) device bytes; sptr: (n + 31) / 32 + 1 entries; info_host: 4
@@ -166,13 +164,14 @@ template <class T>
 void cg_residual(long n, const double* al, const T* q, T* r, T* out, const T* sc, int nsc, T* hsc, T* partial,
                  cudaStream_t s);
 // The kernels from mdot(BU, z) to cg_residual as one launch (one per stream at a time), where the rows and columns
-// allow it: r and p as there, z = B p with B (else left alone), rho (device, this iteration's), and on the host after
-// the stream has synchronised hsc[0..4] = rho, U^H q, BU^H q (with B), p^H q, st.ticket (as the call left it; anything
-// else: a barrier gave up) and hpart[0..g) the partials of r^H r, g the return value, to be added by md_sum_host.
+// allow it: r and p as there, z = B p with B (else left alone), rho (device, this iteration's), and in pinned host
+// memory hsc[0..3] = rho, U^H q, BU^H q (with B), p^H q and hpart[0..g) the partials of r^H r, g the return value, to be
+// added by md_sum_host.  Words still unwritten when the kernel has ended: a barrier gave up; the counter is then to be
+// set to zero, with st.base = 0.
 // part: (k + 3) * reduction_blocks(n) entries; bar: a counter that starts at zero, with st.base = 0, and is only used here.
 struct OneState {
   unsigned base = 0;    // what the barrier counter holds
-  unsigned ticket = 0;  // launches so far
+  int polls = 1 << 22;  // after which a CTA gives up its wait (seconds; a barrier takes a microsecond)
 };
 template <class T> bool inner_one_ok(long n, int k, bool gep);
 constexpr int kMaxPartials = 152 * 8;  // most CTAs of a reduction
