@@ -88,6 +88,8 @@ void build_sell_host(int n, const int* ia, const int* ja, const H* a, SellMatrix
   std::vector<int> cnt(n, 0);
   for (int i = 0; i < n; ++i)
     for (int p = ia[i] - 1; p < ia[i + 1] - 1; ++p) {
+      // the device build checks the row pointers, and the columns of the rows it takes
+      if (ja[p] < 1 || ja[p] > n) throw std::runtime_error("column indices out of range");
       int j = ja[p] - 1;
       cnt[i]++;
       if (j != i) cnt[j]++;

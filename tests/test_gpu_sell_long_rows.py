@@ -31,3 +31,14 @@ def test_row_of_many_stored_entries(gpu, stored, row, cplx):
     size[cols] += np.abs(off) * np.abs(x[hub])
     # a row has at most `stored` terms: that many times eps, twice for complex products and for the two sums
     assert np.all(np.abs(gpu.spmv((a, ja, ia), x) - y) <= 4 * (stored + 4) * np.finfo(float).eps * size + 1e-300)
+
+
+@pytest.mark.parametrize("bad", [0, -5, 6001, 1 << 30])
+@pytest.mark.parametrize("at", [1, 4999])
+def test_bad_column_in_a_long_row_is_refused(gpu, bad, at):
+    n, stored = 6000, 5000
+    ja = np.concatenate([np.arange(1, stored + 1), np.arange(2, n + 1)]).astype(np.int32)
+    ja[at] = bad
+    ia = np.concatenate([[1], np.arange(stored + 1, stored + n + 1)]).astype(np.int32)
+    with pytest.raises(RuntimeError):
+        gpu.spmv((np.ones(len(ja)), ja, ia), np.ones(n))
