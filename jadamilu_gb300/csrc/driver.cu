@@ -82,18 +82,20 @@ template <class T> void sell_slots(SellMatrix<T>& M, int64_t slots) {
   CK(cudaMalloc(&M.val, sizeof(T) * slots));
   M.cap_slots = slots;
 }
-// The host pass: for matrices with a row beyond what the device build takes.
-template <class T, class H>
-void build_sell_host(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, cudaStream_t st) {
+// The host pass: for small matrices (fill_sell) and those with a row beyond what
+// the device build takes; the same checks, the same arrays.
+template <class T, class H, class Room>
+void build_sell_host(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, Room room, cudaStream_t st) {
   std::vector<int> cnt(n, 0);
-  for (int i = 0; i < n; ++i)
+  for (int i = 0; i < n; ++i) {
+    if (ia[i] < 1 || ia[i + 1] < ia[i] || ia[i + 1] > ia[n]) throw std::runtime_error("row pointers out of range");
     for (int p = ia[i] - 1; p < ia[i + 1] - 1; ++p) {
-      // the device build checks the row pointers, and the columns of the rows it takes
       if (ja[p] < 1 || ja[p] > n) throw std::runtime_error("column indices out of range");
       int j = ja[p] - 1;
       cnt[i]++;
       if (j != i) cnt[j]++;
     }
+  }
   std::vector<int64_t> rp(n + 1, 0);
   for (int i = 0; i < n; ++i) rp[i + 1] = rp[i] + cnt[i];
   std::vector<int> ci(rp[n]);
@@ -135,8 +137,7 @@ void build_sell_host(int n, const int* ia, const int* ja, const H* a, SellMatrix
       }
     }
   }
-  sell_slices(M, ns);
-  sell_slots(M, std::max<int64_t>(1, sp[ns]));
+  room(std::max<int64_t>(1, sp[ns]));
   M.nnz = rp[n];
   M.stored = sp[ns];
   CK(cudaMemcpyAsync(M.sptr, sp.data(), sizeof(int64_t) * (ns + 1), cudaMemcpyHostToDevice, st));
@@ -144,34 +145,27 @@ void build_sell_host(int n, const int* ia, const int* ja, const H* a, SellMatrix
   CK(cudaMemcpyAsync(M.val, sval.data(), sizeof(T) * sp[ns], cudaMemcpyHostToDevice, st));
   CK(cudaStreamSynchronize(st));
 }
-// The matrix for the products from the caller's triangle; keep: a staging
-// buffer that outlives the call (a solver's; up to kSellKept bytes), else one
-// of its own.  Returns with the matrix complete: the products load it before
-// they wait for their predecessor, so its writers must not be in flight when
-// one is launched.
-template <class T, class H>
-void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, cudaStream_t st,
-                SellStage* keep = nullptr) {
+// Fills M from the caller's triangle: M.sptr has room for the slices, room(slots)
+// provides M.col and M.val, work is what sell_work_bytes asks for.  The products
+// load a matrix before they wait for their predecessor, so its writers must not
+// be in flight when one is launched: the caller synchronises, or copies.
+// Up to this many stored entries the host pass takes less than the copies and
+// kernels of the device build: a product through the public call, us, host
+// pass and device build (GB300): 81 entries 196 and 230, 1856 215 and 239, 3700
+// 228 and 238, 6480 250 and 242, 15616 318 and 251.
+constexpr int kSellHostEntries = 4096;
+template <class T, class H, class Room>
+void fill_sell(int n, const int* ia, const int* ja, const H* a, void* work, SellMatrix<T>& M, Room room,
+               cudaStream_t st) {
   static_assert(sizeof(T) == sizeof(H), "the values are copied as they are");
-  const int64_t nnz = (int64_t)ia[n] - 1;
-  if (nnz < 0) throw std::runtime_error("row pointers out of range");
-  struct Own : SellStage {
-    ~Own() { release(); }
-  } own;
-  SellStage& stage = keep ? *keep : own;
-  AtExit trim{[&] {
-    if (stage.cap > kSellKept) stage.release();
-  }};
-  const int ns = (n + 31) / 32;
-  // no matrix until its arrays are complete: a refused one leaves foreign slice pointers behind
+  // no matrix until its arrays are there: a refused one leaves foreign slice pointers behind
   M.n = M.nslices = 0;
   M.nnz = M.stored = 0;
-  sell_slices(M, ns);
   unsigned long long info[4] = {};
-  const bool built = k::sell_from_triangle<T>(
-      n, ia, ja, a, stage.need(k::sell_work_bytes(n, nnz, sizeof(T))), M.sptr, info,
+  const bool built = ia[n] - 1 > kSellHostEntries && k::sell_from_triangle<T>(
+      n, ia, ja, a, work, M.sptr, info,
       [&](int64_t slots, int** col, T** val) {
-        sell_slots(M, std::max<int64_t>(1, slots));
+        room(std::max<int64_t>(1, slots));
         *col = M.col;
         *val = M.val;
       },
@@ -179,12 +173,35 @@ void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& 
   if (built) {
     M.stored = (int64_t)info[0];
     M.nnz = (int64_t)info[1];
-    CK(cudaStreamSynchronize(st));
   } else {
-    build_sell_host<T>(n, ia, ja, a, M, st);
+    build_sell_host<T>(n, ia, ja, a, M, room, st);
   }
   M.n = n;
-  M.nslices = ns;
+  M.nslices = (n + 31) / 32;
+}
+static int64_t stored_entries(int n, const int* ia) {
+  if (ia[n] < 1) throw std::runtime_error("row pointers out of range");
+  return (int64_t)ia[n] - 1;
+}
+// The matrix for the products from the caller's triangle, complete on return;
+// keep: a staging buffer that outlives the call (a solver's; up to kSellKept
+// bytes), else one of its own.
+template <class T, class H>
+void build_sell(int n, const int* ia, const int* ja, const H* a, SellMatrix<T>& M, cudaStream_t st,
+                SellStage* keep = nullptr) {
+  const int64_t nnz = stored_entries(n, ia);
+  struct Own : SellStage {
+    ~Own() { release(); }
+  } own;
+  SellStage& stage = keep ? *keep : own;
+  AtExit trim{[&] {
+    if (stage.cap > kSellKept) stage.release();
+  }};
+  M.n = 0;
+  sell_slices(M, (n + 31) / 32);
+  fill_sell<T>(n, ia, ja, a, stage.need(k::sell_work_bytes(n, nnz, sizeof(T))), M,
+               [&](int64_t slots) { sell_slots(M, slots); }, st);
+  CK(cudaStreamSynchronize(st));
 }
 template <class T> void free_sell(SellMatrix<T>& M) {
   void* ps[] = {M.sptr, M.col, M.val};
@@ -1820,18 +1837,28 @@ JDG_API int jdgpu_device_count(void) {
 // y = A x with A given like DPJD's (upper, 1-based); x, y host arrays.
 extern "C++" {
 template <class T, class H> static void spmv_host(int n, const int* ia, const int* ja, const H* a, const H* x, H* y) {
+  // Two allocations, what is known before the build and the matrix's slots, instead
+  // of one per array: 6^3 Laplacian built on the device 245 -> 232 us a call (GB300)
   cudaStream_t st = nullptr;
-  SellMatrix<T> M;
-  T *dx = nullptr, *dy = nullptr;
+  const int64_t work = k::sell_work_bytes(n, stored_entries(n, ia), sizeof(T));
+  const int64_t vec = ((int64_t)sizeof(T) * n + 255) / 256 * 256;
+  unsigned char *fixed = nullptr, *slots = nullptr;
   AtExit gone{[&] {
-    cudaFree(dx);
-    cudaFree(dy);
-    free_sell(M);
+    cudaFree(fixed);
+    cudaFree(slots);
   }};
-  build_sell<T>(n, ia, ja, a, M, st);
-  CK(cudaMalloc(&dx, sizeof(T) * n));
-  CK(cudaMalloc(&dy, sizeof(T) * n));
-  CK(cudaMemcpy(dx, x, sizeof(T) * n, cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&fixed, work + 2 * vec + sizeof(int64_t) * ((n + 31) / 32 + 1)));
+  T *dx = (T*)(fixed + work), *dy = (T*)(fixed + work + vec);
+  SellMatrix<T> M;  // borrows its arrays
+  M.sptr = (int64_t*)(fixed + work + 2 * vec);
+  fill_sell<T>(n, ia, ja, a, fixed, M,
+               [&](int64_t count) {
+                 CK(cudaMalloc(&slots, count * (int64_t)(sizeof(T) + sizeof(int))));
+                 M.val = (T*)slots;
+                 M.col = (int*)(slots + count * (int64_t)sizeof(T));
+               },
+               st);
+  CK(cudaMemcpy(dx, x, sizeof(T) * n, cudaMemcpyHostToDevice));  // orders the build before the product
   k::spmv<T>(M, dx, dy, st);
   CK(cudaGetLastError());
   CK(cudaMemcpy(y, dy, sizeof(T) * n, cudaMemcpyDeviceToHost));
