@@ -395,7 +395,7 @@ correction:
       const bool POSDEF = (IFO == 1);
       IFO = 0;
       const int MAXIT = ITCG;
-      double GGK2 = GK * GK, RHO = 0, RHO1 = 0, TTK2 = 0, TTK2M = 0;
+      double GGK2 = GK * GK, RHO = 0, TTK2 = 0, TTK2M = 0;
       int it = 0;
       bool fail = false;
       // RHO of iteration `it` is kept in device slot kScal + (it & 1), so the
@@ -405,14 +405,13 @@ correction:
       for (;;) {
         ++it;
         // RHO, the projection coefficient, the B-inner product, P^H Q and |R|^2
-        // stay on the device and are read back together: one synchronisation
-        // per iteration with the built-in operators (in one kernel beside the
-        // preconditioner, k::inner_one, where the size allows it), one more
-        // before a caller's matvec, which is not asked for when RHO ends the
-        // solve.  A check that fails after the read leaves Q, Z and R (and P
-        // after the first iteration) modified where a sequence with a read
-        // per scalar stops earlier; none of them is read after a failed inner
-        // solve.
+        // are read by the host together: one wait per iteration with the
+        // built-in operators (in one kernel beside the preconditioner,
+        // k::inner_one, where the size allows it), one more before a caller's
+        // matvec, which is not asked for when RHO ends the solve.  A check that
+        // fails after the read leaves Q, Z and R (and P after the first
+        // iteration) modified where a sequence with a read per scalar stops
+        // earlier; none of them is read after a failed inner solve.
         precond(R, Zv);
         S_.flagcg = true;
         T* rho_d = scd + (it & 1);
@@ -506,7 +505,6 @@ correction:
         FTFLG = false;
         if (IFO == 1) { IFO = 0; break; }
         if (it == MAXIT) { fail = true; break; }
-        RHO1 = RHO;
       }
       if (fail) {
         IFO = 1;

@@ -7,7 +7,8 @@
 // (NDX1/NDX2/NDX3) and the eigenvector output keep their meaning.  The J x J
 // projected matrices and the small coefficient vectors stay in the caller's
 // host X at the same offsets.  Scalars that steer the control flow (norms,
-// inner products) are read back with one stream synchronisation each.
+// inner products) are written to pinned host words by the kernels that form
+// them; the host watches those words (DevJd::await).
 #pragma once
 #include <cfloat>
 #include <chrono>

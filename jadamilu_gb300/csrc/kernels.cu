@@ -1573,14 +1573,10 @@ __global__ void __launch_bounds__(RUN_TPB) ildl_run_kernel(int l0, int l1, const
 // the successor's blocks, there to load their entries, otherwise take turns on
 // the FP64 units and slots this level still needs.  us per application (GB300),
 // 256 threads and early -> as here: FEM 384^2 float64 276 -> 238, tight-binding
-// 48^3 complex128 386 -> 277, complex64 139 -> 132, Anderson 44^3 float64 361 ->
-// 340, Laplacian 32^3 185 -> 181; early with 128 threads 268, 375, -, 357, 183;
-// float32 late: FEM 127.6 -> 131.5, Anderson 44^3 155.6 -> 156.8.  A float64 tile
+// 48^3 complex128 386 -> 277, Anderson 44^3 float64 361 -> 340; float32, were it
+// late as well: FEM 127.6 -> 131.5, Anderson 44^3 155.6 -> 156.8.  A float64 tile
 // product (tri_cluster_kernel) lets it start once its products are done: FEM
-// 384^2 239 -> 232, Anderson 36^3 269 -> 261.5, a FEM 512^2 solve 214.5 -> 211.1
-// ms, Laplacian 20^3 30.2 -> 29.7.  A level that waits for its products, too, is
-// faster when applications follow one another (FEM 384^2 238 -> 234) but not in a
-// solve (FEM 512^2 226.9 ms): its successor then asks for its entries too late.
+// 384^2 239 -> 232, a FEM 512^2 solve 214.5 -> 211.1 ms.
 constexpr int WIDE_TPB = 128;
 template <class A> constexpr bool kLate = sizeof(A) == 16 || std::is_same<A, double>::value;
 static inline int lanes_for(double entries_per_row) {
@@ -1808,10 +1804,7 @@ __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
 // application (GB300), one tile at a time with the rest of the chunk
 // prefetched into L2 -> now: Laplacian 20^3 float64 72.2 -> 69.0, Anderson
 // 28^3 float64 205.7 -> 166.6, float32 70.3 -> 67.5, 40^3 186.6 -> 162.1, 56^3
-// 431 -> 375, 25^3 bfloat16 46.1 -> 47.3.  Two units in flight: 71.8, 172.2,
-// 67.4, 160.3, 377.9, 48.8; three with the prefetch: 69.1, 174.0, 64.6, 178.2,
-// 389.3, 46.3.  Bulk copies through shared memory (four 16 KB stages) were
-// slower for float32 (40^3 201, 56^3 506): the stages cost resident CTAs.
+// 431 -> 375, 25^3 bfloat16 46.1 -> 47.3.
 template <class S, class A, int CL>
 __global__ void __launch_bounds__(TRI_TPB)
     tri_cluster_kernel(const int4* __restrict__ items, bool rev, const S* __restrict__ tiles, const A* __restrict__ x,

@@ -92,7 +92,7 @@ template <class S> struct DevFactor {
   // one CSR over all steps) and, per level l, F_l^H (rows: the steps after
   // level l, row pointers from fhp + fh_row0[l]; columns: the level's steps),
   // and three outer-precision work vectors of n entries.  The fields above
-  // then hold only n, nnz_l, graph and the graph's input/output vectors.
+  // then hold only n, nnz_l and the graph with its nodes and vectors.
   int coupled = 0;
   std::vector<DevFactor<S>> lev;
   std::vector<int> lstart;                   // first step of each level, plus n
