@@ -204,7 +204,9 @@ JDG_API int jdgpu_dildl_bench(int n, const int* ia, const int* ja, const double*
 
 /* Device-resident mode (no reference counterpart; used for repeated solves
  * and timing): upload A once, let dpjd_ reuse it and keep eigenvectors on the
- * device, until jdgpu_drelease_matrix(). */
+ * device, until jdgpu_drelease_matrix().  A refused matrix leaves none
+ * prepared; a solve of another size ends with INFO = -54330; dpjd_gep_ hands
+ * its B over by itself. */
 JDG_API int jdgpu_dprepare_matrix(int n, const int* ia, const int* ja, const double* a);
 JDG_API void jdgpu_drelease_matrix(void);
 JDG_API void jdgpu_dmatrix_info(long* out);

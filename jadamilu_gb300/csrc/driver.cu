@@ -180,7 +180,7 @@ void fill_sell(int n, const int* ia, const int* ja, const H* a, void* work, Sell
   M.nslices = (n + 31) / 32;
 }
 static int64_t stored_entries(int n, const int* ia) {
-  if (ia[n] < 1) throw std::runtime_error("row pointers out of range");
+  if (n < 0 || ia[n] < 1) throw std::runtime_error("row pointers out of range");
   return (int64_t)ia[n] - 1;
 }
 // The matrix for the products from the caller's triangle, complete on return;
@@ -725,7 +725,7 @@ template <class T> struct Global {
   double* ddiag = nullptr; // diagonal preconditioner on the device
   SellMatrix<T> A, Bm;     // built-in matvec operands
   SellStage stage;         // and the buffer they are built from
-  bool resident = false;   // A (and B) prepared on the device by the caller
+  bool resident = false;   // A prepared on the device by the caller
   int nfactor = 0;
   double t_factor = 0, t_upload = 0;
   long n_precond = 0, n_matvec = 0;
@@ -1239,9 +1239,13 @@ void pjd_drive(int n, typename HostOf<T>::type* a, int* ja, int* ia, typename Ho
   }
   const double t1 = wall();
   // operands of the built-in matvec
-  if (!user_mv && !g.resident) {
-    if (ja[0] < 0) throw std::runtime_error("diagonal preconditioning needs the reverse-communication matvec");
-    build_sell<T>(n, ia, ja, a, g.A, g.W.st, &g.stage);
+  if (!user_mv) {
+    if (!g.resident) {
+      if (ja[0] < 0) throw std::runtime_error("diagonal preconditioning needs the reverse-communication matvec");
+      build_sell<T>(n, ia, ja, a, g.A, g.W.st, &g.stage);
+    } else if (g.A.n != n) {  // the product kernels take one size for all vectors
+      throw std::runtime_error("the prepared matrix has another size");
+    }
     if (gep) build_sell<T>(n, ib, jb, b, g.Bm, g.W.st, &g.stage);
   }
   // initial guesses

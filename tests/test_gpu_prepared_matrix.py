@@ -68,3 +68,37 @@ def test_stream_replaced_between_prepare_and_solve(gpu):
     finally:
         gpu.set_stream(0)
         gpu.release_matrix()
+
+
+def test_generalized_solves_with_a_prepared_matrix(gpu):
+    """Only A is prepared: every generalized solve hands its own B over, after
+    one of a smaller size and after one with another B."""
+    def pencil(m, seed):
+        K, B = M.fem_p1(m, seed=seed)
+        return (K[2], K[1], K[0]), (B[2], B[1], B[0])
+
+    small = pencil(20, 3)
+    A, B = pencil(100, 3)
+    B2 = (2.0 * B[0], B[1], B[2])
+    plain = [gpu.dpjd_gep(A, Bk, 3, **KW)["eigs"] for Bk in (B, B2)]
+    assert gpu.dpjd_gep(*small, 3, **KW)["info"] == 0
+    try:
+        gpu.prepare_matrix(A)
+        for Bk, w in zip((B, B2), plain):
+            r = gpu.dpjd_gep(A, Bk, 3, **KW)
+            assert r["info"] == 0
+            np.testing.assert_array_equal(r["eigs"], w)
+    finally:
+        gpu.release_matrix()
+
+
+def test_solve_of_another_size_is_refused(gpu):
+    ia, ja, a = M.laplace3d(12)
+    try:
+        gpu.prepare_matrix((a, ja, ia))
+        for m in (10, 14):
+            ib, jb, b = M.laplace3d(m)
+            assert gpu.dpjd((b, jb, ib), 3, **KW)["info"] == -54330
+        assert gpu.dpjd((a, ja, ia), 3, **KW)["info"] == 0
+    finally:
+        gpu.release_matrix()
