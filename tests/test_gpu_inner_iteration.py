@@ -58,3 +58,24 @@ def test_batch_of_problems_with_grid_barriers(gpu):
     for r, w in zip(gpu.dpjd_batch(problems, 4, workers=8, isearch=0, tol=tol, icntl=(0, 0, 0, 0, 0)), exact):
         assert r["info"] == 0 and r["neig"] == 4
         assert np.max(np.abs(np.sort(r["eigs"]) - w)) <= tol + 64 * np.finfo(float).eps * 12 * 2.5
+
+
+@pytest.mark.parametrize("n", [4096, 8193, 77825])
+@pytest.mark.parametrize("kind,isearch", [("real", 2), ("complex generalized", 2)])
+def test_most_columns(gpu, n, kind, isearch):
+    """32 pairs, the most that the drivers sort: up to 32 columns in a projection."""
+    A, B = _problem(kind, n)
+    got = []
+    for fuse in (1, 0):
+        gpu.set_option("fuse_inner", fuse)
+        try:
+            kw = dict(isearch=isearch, sigma=0.0, madspace=20, maxit=20000, tol=1e-9, droptol=1e-3,
+                      icntl=(0, 1, 0, 0, 0))
+            r = gpu.dpjd(A, 32, **kw) if B is None else gpu.zpjd_gep(A, B, 32, **kw)
+        finally:
+            gpu.set_option("fuse_inner", 1)
+        assert r["info"] == 0 and r["neig"] == 32
+        got.append(r)
+    assert got[0]["iter"] == got[1]["iter"]
+    for key in ("eigs", "res", "x"):
+        np.testing.assert_array_equal(got[0][key], got[1][key])
